@@ -134,7 +134,7 @@ class CqaBatchItem(C.Structure):
 class CqaPrefillItem(C.Structure):
     _fields_ = [
         ("cache", CqaCache), ("k_src", vp), ("v_src", vp), ("src_rows", C.c_int64), ("n_tokens", C.c_int64),
-        ("defer_int4", C.c_int32), ("reserved", C.c_int32),
+        ("defer_int4", C.c_int32), ("init_reserve", C.c_int32),
     ]
 
 

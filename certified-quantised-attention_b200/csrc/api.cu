@@ -91,12 +91,12 @@ extern "C" const char *cqa_last_error(void) { return g_err; }
 extern "C" int cqa_wait_timeouts(int *count, int reset)
 {
     if (!count) { set_error("cqa_wait_timeouts: NULL pointer"); return CQA_ERR_INVALID; }
-    int a = 0, b = 0;
-    if (score_wait_timeouts(&a, reset) || selcert_wait_timeouts(&b, reset)) {
+    int a = 0, b = 0, e = 0;
+    if (score_wait_timeouts(&a, reset) || selcert_wait_timeouts(&b, reset) || quantize_wait_timeouts(&e, reset)) {
         set_error("cqa_wait_timeouts: could not read the device counters: %s", cudaGetErrorString(cudaGetLastError()));
         return CQA_ERR_CUDA;
     }
-    *count = a + b;
+    *count = a + b + e;
     return CQA_OK;
 }
 

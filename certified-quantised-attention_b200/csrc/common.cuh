@@ -486,6 +486,7 @@ int check_score_args(const cqa_cache *c, int q_dtype, long nq, long ld, const ch
 int selcert_check(const cqa_cache *c, const cqa_knobs *kn, const cqa_workspace *ws, const void *q, long nq, int phases);
 int attend_check(const cqa_cache *c, const cqa_workspace *ws, long nq, long nact, int last_valid);
 int append_check(const cqa_cache *c, const void *k_new, const void *v_new, int src_dtype, long pos);
+int quantize_wait_timeouts(int *count, int reset);
 int score_wait_timeouts(int *count, int reset);
 int selcert_wait_timeouts(int *count, int reset);
 

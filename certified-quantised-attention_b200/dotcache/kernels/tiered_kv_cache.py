@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import ctypes as C
 from collections import OrderedDict
+from collections.abc import Mapping
 from dataclasses import dataclass, field
 from typing import Any
 
@@ -37,6 +38,26 @@ def _require_cuda(t: torch.Tensor, what: str) -> None:
             f"{what} must be a CUDA tensor: this cache runs only on the GPU library "
             "(libcqa_b200.so); there is no CPU fallback"
         )
+
+
+class _IdentityResidency(Mapping):
+    """block -> slot of a full mirror: n blocks, each in its own slot."""
+
+    __slots__ = ("n",)
+
+    def __init__(self, n: int):
+        self.n = int(n)
+
+    def __getitem__(self, block):
+        if 0 <= block < self.n:
+            return block
+        raise KeyError(block)
+
+    def __iter__(self):
+        return iter(range(self.n))
+
+    def __len__(self):
+        return self.n
 
 
 @dataclass
@@ -71,13 +92,13 @@ class TieredKeyCacheLayer:
     values_fp16_cpu: torch.Tensor | None = None
     values_fp16_gpu: torch.Tensor | None = None
     fp16_value_cache_capacity: int | None = None
-    _fp16_value_resident: "OrderedDict[int, int]" = field(default_factory=OrderedDict)
+    _fp16_value_resident: Mapping = field(default_factory=OrderedDict)
     _fp16_value_free_slots: list = field(default_factory=list)
     static_resident_value_cache: bool = False
     static_resident_value_prepare_bytes: int = 0
     keys_fp16_gpu: torch.Tensor | None = None
     fp16_key_cache_capacity: int | None = None
-    _fp16_key_resident: "OrderedDict[int, int]" = field(default_factory=OrderedDict)
+    _fp16_key_resident: Mapping = field(default_factory=OrderedDict)
     _fp16_key_free_slots: list = field(default_factory=list)
     static_resident_key_cache: bool = False
     static_resident_key_prepare_bytes: int = 0
@@ -149,8 +170,10 @@ class TieredKeyCacheLayer:
 
     @classmethod
     def _allocate(cls, keys: torch.Tensor, values: torch.Tensor, block_size: int, max_pagein_blocks: int,
-                  max_new_tokens: int, int4: bool, group_size: int,
-                  hot_blocks: tuple[int, int] | None = None) -> "TieredKeyCacheLayer":
+                  max_new_tokens: int, int4: bool, group_size: int, hot_blocks: tuple[int, int] | None = None,
+                  sigma_max: torch.Tensor | None = None) -> "TieredKeyCacheLayer":
+        """The cache's arrays.  A full mirror's are left uninitialised: the encode that follows writes the prompt and
+        sets the capacity behind it to the empty state (`init_reserve`), one launch in place of a fill per array."""
         _require_cuda(keys, "keys")
         _require_cuda(values, "values")
         if block_size != BLOCK:
@@ -171,20 +194,21 @@ class TieredKeyCacheLayer:
         cap = N + max_new_tokens
         maxblk = nb + (max_new_tokens + BLOCK - 1) // BLOCK
         kvd = keys.dtype
-        z = torch.zeros
+        z = torch.empty if hot_blocks is None else torch.zeros
+        f32 = dict(dtype=torch.float32, device=dev)
         self = cls(
             keys_int8=z(kv, cap, hd, dtype=torch.int8, device=dev),
-            keys_scale=z(kv, maxblk, hd, dtype=torch.float32, device=dev),
-            keys_zero_points=z(kv, maxblk, hd, dtype=torch.float32, device=dev),
-            correction=torch.ones(kv, maxblk, dtype=torch.float32, device=dev),
+            keys_scale=z(kv, maxblk, hd, **f32),
+            keys_zero_points=z(kv, maxblk, hd, **f32),
+            correction=torch.empty(kv, maxblk, **f32) if hot_blocks is None else torch.ones(kv, maxblk, **f32),
             values_fp16=None,
             keys_fp16_cpu=None,
             kv_heads=kv, num_tokens=N, head_dim=hd, d_v=dv, block_size=BLOCK, num_blocks=nb,
             num_quantized_blocks=nb,
             _pagein_buffer=torch.empty(max_pagein_blocks * BLOCK, hd, dtype=kvd, device=dev),
-            values_norm_max_per_block=z(kv, maxblk, dtype=torch.float32, device=dev),
+            values_norm_max_per_block=z(kv, maxblk, **f32),
             keys_fp16_gpu=z(kv, cap if hot_blocks is None else hot_blocks[0] * BLOCK, hd, dtype=kvd, device=dev),
-            keys_scale_max=z(kv, hd, dtype=torch.float32, device=dev),
+            keys_scale_max=torch.zeros(kv, hd, **f32) if sigma_max is None else sigma_max,
         )
         vbuf = z(kv, cap if hot_blocks is None else hot_blocks[1] * BLOCK, dv, dtype=kvd, device=dev)
         if hot_blocks is not None:
@@ -215,27 +239,18 @@ class TieredKeyCacheLayer:
             self.values_int4_packed = z(kv, cap, dv // 2, dtype=torch.uint8, device=dev)
             self.values_int4_scales = z(kv, cap, dv // 16, dtype=torch.float16, device=dev)
             self.values_int4_zeros = z(kv, cap, dv // 16, dtype=torch.float16, device=dev)
-            self.values_int4_errors = z(kv, maxblk, dtype=torch.float32, device=dev)
-            self.values_int4_error_sums = z(kv, maxblk, dtype=torch.float32, device=dev)
+            self.values_int4_errors = z(kv, maxblk, **f32)
+            self.values_int4_error_sums = z(kv, maxblk, **f32)
             self.values_int4_error_counts = z(kv, maxblk, dtype=torch.int32, device=dev)
             self.values_int4_group_size = 16
             self.values_fp16_gpu = vbuf
         else:
             self.values_fp16 = vbuf
-        self._fp16_key_resident = OrderedDict((i, i) for i in range(nb))
+        self._fp16_key_resident = _IdentityResidency(nb)
         return self
 
     def _quantize_prefill(self, keys: torch.Tensor, values: torch.Tensor) -> None:
-        N = keys.shape[1]
-        if N == 0:
-            return
-        keys = keys.contiguous()
-        values = values.to(keys.dtype).contiguous()
-        with torch.cuda.device(keys.device):
-            rc = _lib.lib().cqa_quantize_blocks(
-                C.byref(self._desc()), keys.data_ptr(), values.data_ptr(), _lib.dtype_code(keys.dtype),
-                N, 0, N // BLOCK, _lib.current_stream(keys.device))
-        _lib.check(rc, "cqa_quantize_blocks")
+        _encode_prefill_layers([(self, keys, values, keys.shape[1])])
 
     @staticmethod
     def _check_capacity(cap, max_blocks: int, what: str):
@@ -248,11 +263,12 @@ class TieredKeyCacheLayer:
     @classmethod
     def from_fp16_cache(cls, keys_fp16: torch.Tensor, values_fp16: torch.Tensor, block_size: int = 16,
                         max_pagein_blocks: int = 64, max_new_tokens: int = 512,
-                        fp16_key_cache_capacity: int | None = None, _encode: bool = True) -> "TieredKeyCacheLayer":
+                        fp16_key_cache_capacity: int | None = None, _encode: bool = True,
+                        _sigma_max: torch.Tensor | None = None) -> "TieredKeyCacheLayer":
         """INT8 keys + model-dtype values (reference: tiered_kv_cache.py:135-286).  `_encode=False` only allocates
         (the whole-model constructors encode every layer in one library call afterwards)."""
         self = cls._allocate(keys_fp16, values_fp16, block_size, max_pagein_blocks, max_new_tokens,
-                             int4=False, group_size=16)
+                             int4=False, group_size=16, sigma_max=_sigma_max)
         cap = cls._check_capacity(fp16_key_cache_capacity, self.keys_scale.shape[1], "fp16_key_cache_capacity")
         if cap is not None and cap < self.keys_scale.shape[1]:
             raise NotImplementedError(
@@ -263,7 +279,7 @@ class TieredKeyCacheLayer:
         if cap is not None:
             self.fp16_key_cache_capacity = cap
             self.static_resident_key_cache = True
-            self._fp16_key_resident = OrderedDict((i, i) for i in range(self.keys_scale.shape[1]))
+            self._fp16_key_resident = _IdentityResidency(self.keys_scale.shape[1])
         return self
 
     @classmethod
@@ -272,7 +288,7 @@ class TieredKeyCacheLayer:
                               fp16_key_cache_capacity: int | None = None,
                               fp16_value_cache_capacity: int | None = None,
                               defer_int4_append_quantization: bool = False,
-                              _encode: bool = True) -> "TieredKeyCacheLayer":
+                              _encode: bool = True, _sigma_max: torch.Tensor | None = None) -> "TieredKeyCacheLayer":
         """INT8 keys + INT4 g16 values (reference: tiered_kv_cache.py:289-405).  `_encode=False` only allocates."""
         nb0 = keys_fp16.shape[1] // BLOCK
         maxblk = nb0 + (max_new_tokens + BLOCK - 1) // BLOCK
@@ -286,7 +302,7 @@ class TieredKeyCacheLayer:
             hot_blocks = (min(kcap, maxblk) if kcap is not None else maxblk,
                           min(vcap, maxblk) if vcap is not None else maxblk)
         self = cls._allocate(keys_fp16, values_fp16, block_size, max_pagein_blocks, max_new_tokens,
-                             int4=True, group_size=group_size, hot_blocks=hot_blocks)
+                             int4=True, group_size=group_size, hot_blocks=hot_blocks, sigma_max=_sigma_max)
         if bounded:
             self.defer_int4_append_quantization = bool(defer_int4_append_quantization)
             if _encode:
@@ -300,7 +316,7 @@ class TieredKeyCacheLayer:
         if kcap is not None:
             self.fp16_key_cache_capacity = kcap
             self.static_resident_key_cache = True
-            self._fp16_key_resident = OrderedDict((i, i) for i in range(maxblk))
+            self._fp16_key_resident = _IdentityResidency(maxblk)
         if vcap is not None:
             # A capacity that covers the reserved context is the reference's
             # "static resident" mode, which also defers INT4 append
@@ -308,7 +324,7 @@ class TieredKeyCacheLayer:
             self.fp16_value_cache_capacity = vcap
             self.static_resident_value_cache = True
             self.defer_int4_append_quantization = True
-            self._fp16_value_resident = OrderedDict((i, i) for i in range(maxblk))
+            self._fp16_value_resident = _IdentityResidency(maxblk)
         return self
 
     # ------------------------------------------------------------------ append
@@ -536,6 +552,15 @@ def _layer_kv(past_kv, layer_id: int, batch_index: int = 0):
     return past_kv[layer_id][0][batch_index], past_kv[layer_id][1][batch_index]
 
 
+def _layer_sigma_max(past_kv, layer_ids: list, batch_index: int = 0):
+    """The layers' running channel maxima, zeroed by one fill (None per layer when the layers differ in heads or device)."""
+    shapes = {(k.shape[0], k.shape[2], k.device) for k in (_layer_kv(past_kv, l, batch_index)[0] for l in layer_ids)}
+    if len(shapes) != 1:
+        return [None] * len(layer_ids)
+    kv, hd, dev = shapes.pop()
+    return torch.zeros(len(layer_ids), kv, hd, dtype=torch.float32, device=dev).unbind(0)
+
+
 def _encode_prefill_layers(entries) -> None:
     """entries: (cache, keys [KV, seq, 128], values, seq_len) per layer, caches allocated but empty.  One library
     call per (device, dtype) group quantises every layer's complete blocks straight from the prefill tensors and
@@ -559,9 +584,11 @@ def _encode_prefill_layers(entries) -> None:
         items = (_lib.CqaPrefillItem * len(group))()
         for i, (cache, keys, values, seq_len, rows) in enumerate(group):
             items[i].cache = cache._desc()
-            items[i].k_src = keys.data_ptr()
-            items[i].v_src = values.data_ptr()
+            # an empty prompt has no memory of its own; nothing is read from it
+            items[i].k_src = keys.data_ptr() or cache.keys_int8.data_ptr()
+            items[i].v_src = values.data_ptr() or cache.keys_int8.data_ptr()
             items[i].src_rows = rows
+            items[i].init_reserve = 0 if cache.bounded_hot_tier else 1
             items[i].n_tokens = seq_len
             items[i].defer_int4 = 1 if cache._defer_int4_flag() else 0
         with _lib.on_device(dev):
@@ -585,7 +612,8 @@ def create_tiered_cache_int4v_from_model(past_kv, layer_ids: list, block_size: i
     if defer_int4_append_quantization is None:
         defer_int4_append_quantization = fp16_value_cache_capacity is None
     caches, entries = {}, []
-    for layer_id in layer_ids:
+    sigma = _layer_sigma_max(past_kv, layer_ids, batch_index)
+    for layer_id, sigma_max in zip(layer_ids, sigma):
         keys, values = _layer_kv(past_kv, layer_id, batch_index)
         seq_len = keys.shape[1]
         aligned = (seq_len // block_size) * block_size
@@ -595,7 +623,7 @@ def create_tiered_cache_int4v_from_model(past_kv, layer_ids: list, block_size: i
             max_new_tokens=max_new_tokens + (seq_len - aligned),
             fp16_key_cache_capacity=fp16_key_cache_capacity,
             fp16_value_cache_capacity=fp16_value_cache_capacity,
-            defer_int4_append_quantization=bool(defer_int4_append_quantization), _encode=False,
+            defer_int4_append_quantization=bool(defer_int4_append_quantization), _encode=False, _sigma_max=sigma_max,
         )
         cache.num_tokens = cache.num_blocks = cache.num_quantized_blocks = 0
         entries.append((cache, keys, values, seq_len))
@@ -608,14 +636,15 @@ def create_tiered_cache_from_model(past_kv, layer_ids: list, block_size: int = 1
                                    fp16_key_cache_capacity: int | None = None) -> dict:
     """Per-layer INT8-key / model-dtype-value caches (reference: tiered_kv_cache.py:1644-1701)."""
     caches, entries = {}, []
-    for layer_id in layer_ids:
+    sigma = _layer_sigma_max(past_kv, layer_ids)
+    for layer_id, sigma_max in zip(layer_ids, sigma):
         keys, values = _layer_kv(past_kv, layer_id)
         seq_len = keys.shape[1]
         aligned = (seq_len // block_size) * block_size
         cache = TieredKeyCacheLayer.from_fp16_cache(
             keys[:, :aligned, :], values[:, :aligned, :],
             block_size=block_size, max_new_tokens=max_new_tokens + (seq_len - aligned),
-            fp16_key_cache_capacity=fp16_key_cache_capacity, _encode=False,
+            fp16_key_cache_capacity=fp16_key_cache_capacity, _encode=False, _sigma_max=sigma_max,
         )
         cache.num_tokens = cache.num_blocks = cache.num_quantized_blocks = 0
         entries.append((cache, keys, values, seq_len))
