@@ -19,6 +19,7 @@ import ctypes as C
 import math
 from typing import Any
 
+import numpy as np
 import torch
 
 from cqa_b200 import _lib
@@ -34,6 +35,7 @@ DEFAULT_RUNG1_MULTIPLIER = 2.0
 
 _CERT_INT_FIELDS = [f for f, t in _lib.CqaHeadCert._fields_ if t is C.c_int32]
 _CERT_F32_FIELDS = [f for f, t in _lib.CqaHeadCert._fields_ if t is C.c_float]
+_CERT_DTYPE = np.dtype(_lib.CqaHeadCert)
 
 
 # ----------------------------------------------------------------------------- workspace
@@ -80,10 +82,11 @@ class _Workspace:
         self.dense_m = torch.empty(H, self.dense_splits, **f32)
         self.dense_l = torch.empty(H, self.dense_splits, **f32)
         self.dense_acc = torch.empty(H, self.dense_splits, 128, **f32)
-        # certificate structs followed by the flag words (4 flags, dense-head count and list):
-        # one D2H copy reads both
+        # certificate structs, the flag words (4 flags, dense-head count and list) and the telemetry words of
+        # cqa_step_stats: one D2H copy reads all three
         self.cert_bytes = H * _lib.CERT_BYTES
-        self.cert_buf = torch.zeros(self.cert_bytes + 4 * (5 + H), **u8)
+        self.stats_off = self.cert_bytes + 4 * (5 + H)
+        self.cert_buf = torch.zeros(self.stats_off + 4 * (2 * H + 2 * cache.kv_heads + _lib.STATS_PARTS), **u8)
         self.out = torch.empty(H, 128, **f32)
         self.tickets = torch.zeros(cache.kv_heads + H, dtype=torch.int32, device=device)
         self.cert_host = None
@@ -155,19 +158,27 @@ class _Workspace:
             object.__setattr__(self, "_struct_stale", True)
         object.__setattr__(self, name, value)
 
+    def _read_back(self) -> np.ndarray:
+        """The certificate buffer on the host (synchronises), through a pinned buffer that is kept."""
+        buf = self.cert_buf
+        host = self.cert_host
+        if host is None or host.numel() != buf.numel():
+            host = self.cert_host = torch.empty(buf.numel(), dtype=torch.uint8, pin_memory=True)
+        host.copy_(buf, non_blocking=True)
+        torch.cuda.current_stream(buf.device).synchronize()
+        return host.numpy()
+
     def read_cert(self) -> tuple[dict, list]:
         """Copy the certificate structs and flags to the host (synchronises)."""
-        host = self.cert_buf.cpu().numpy()
-        arr = (_lib.CqaHeadCert * self.H).from_buffer_copy(host[: self.cert_bytes].tobytes())
-        import numpy as np
-
-        flags = np.frombuffer(host[self.cert_bytes:].tobytes(), dtype=np.int32).tolist()
-        cols: dict[str, Any] = {}
-        for f in _CERT_INT_FIELDS + _CERT_F32_FIELDS:
-            cols[f] = np.array([getattr(arr[h], f) for h in range(self.H)])
-        cols["top_blocks"] = np.array([list(arr[h].top_blocks) for h in range(self.H)])
-        cols["fp16_scores"] = np.array([list(arr[h].fp16_scores) for h in range(self.H)], dtype=np.float32)
-        cols["fp16_logmass"] = np.array([list(arr[h].fp16_logmass) for h in range(self.H)], dtype=np.float32)
+        host = self._read_back()
+        arr = np.frombuffer(host[: self.cert_bytes].tobytes(), dtype=_CERT_DTYPE)
+        flags = np.frombuffer(host[self.cert_bytes: self.stats_off].tobytes(), dtype=np.int32).tolist()
+        cols: dict[str, Any] = {f: arr[f].astype(np.int64) for f in _CERT_INT_FIELDS}
+        for f in _CERT_F32_FIELDS:
+            cols[f] = arr[f].astype(np.float64)
+        cols["top_blocks"] = arr["top_blocks"].astype(np.int64)
+        cols["fp16_scores"] = arr["fp16_scores"].copy()
+        cols["fp16_logmass"] = arr["fp16_logmass"].copy()
         return cols, flags
 
 
@@ -791,23 +802,35 @@ def _assemble_stats(cache, ws: _Workspace, H, G, nq, nact, *, has_int4, force_tr
                     rung1_threshold, rung1_multiplier, exploration_rate, score_consistency_check, eps_guard,
                     ranking_fallback, ranking_r, ranking_fallback_mode, top_k_fp16_keys,
                     value_error_mode) -> dict[str, Any]:
-    """The reference's per-layer stats dict (certified_attention.py:2608-2788)."""
-    import numpy as np
-
-    cert, flags = ws.read_cert()
-    rung4 = bool(score_consistency_check and flags[2])
+    """The reference's per-layer stats dict (certified_attention.py:2608-2788).  One telemetry kernel behind the step
+    and one copy of the certificate buffer; everything after that is host arithmetic on short lists."""
+    KV = cache.kv_heads
+    dev = ws.cert_buf.device
+    with _lib.on_device(dev):
+        _lib.check(_lib.lib().cqa_step_stats(C.byref(cache._desc(G)), C.byref(ws.struct), nq, nact,
+                                             ws.cert_buf.data_ptr() + ws.stats_off, _lib.current_stream(dev)),
+                   "cqa_step_stats")
+    host = ws._read_back()
+    arr = np.frombuffer(host, dtype=_CERT_DTYPE, count=H)
+    flag2 = int(host[ws.cert_bytes + 8: ws.cert_bytes + 12].view(np.int32)[0])
+    tele_i = host[ws.stats_off:].view(np.int32)
+    tele_f = host[ws.stats_off:].view(np.float32)
+    col = lambda name: arr[name].tolist()  # noqa: E731
+    mean = lambda v: sum(v) / len(v)  # noqa: E731
+    rung4 = bool(score_consistency_check and flag2)
     kb, vb = _vram_stats(cache)
     total_blocks = H * cache.num_blocks
-    violation_heads = int(cert["consistency_violation"].sum())
-    boundary_heads = int(cert["boundary_triggered"].sum())
-    rung1_heads = int(cert["rung1_triggered"].sum())
+    delta = col("delta")
+    violation_heads = sum(col("consistency_violation"))
+    boundary_heads = sum(col("boundary_triggered"))
+    rung1_heads = sum(col("rung1_triggered"))
     if rung4:
         # every head was recomputed densely; same keys as the reference's early return (:1771-1796)
         return {
             "total_blocks": total_blocks, "skipped_blocks": 0, "skip_rate": 0.0,
             "attended_blocks": total_blocks, "v_format": "fp16",
             "score_consistency_violation_heads": violation_heads,
-            "delta_bound_mean": float(cert["delta"].mean()), "eps_guard": float(eps_guard),
+            "delta_bound_mean": mean(delta), "eps_guard": float(eps_guard),
             "h2d_key_bytes": 0, "h2d_key_blocks": 0, "h2d_value_bytes": 0, "h2d_value_blocks": 0,
             "h2d_total_bytes": 0, "vram_fp16_key_cache_bytes": kb, "vram_fp16_value_cache_bytes": vb,
             "rung1_fired": bool(rung1_heads > 0), "rung2_fired": False, "rung3_fired": False,
@@ -815,16 +838,15 @@ def _assemble_stats(cache, ws: _Workspace, H, G, nq, nact, *, has_int4, force_tr
             "boundary_check_triggered_heads": boundary_heads,
             "boundary_check_fired": bool(boundary_heads > 0),
         }
-    skipped = int((ws.topk_mask[:, :nact] == 0).sum().item())
-    vmask_q = ws.value_mask[:, :nq]
-    head_blocks = int(cert["value_promoted_blocks"].sum()) if has_int4 else 0
-    union_blocks = int((vmask_q.amax(dim=0) > 0).sum().item()) if (has_int4 and head_blocks) else 0
+    skipped = int(tele_i[:H].sum())
+    head_blocks = sum(col("value_promoted_blocks")) if has_int4 else 0
+    union_blocks = int(tele_i[2 * H + 2 * KV:].sum()) if (has_int4 and head_blocks) else 0
     if has_int4:
         v_format = "mixed" if (head_blocks or force_trailing) else "int4"
     else:
         v_format = "fp16"
     rung2 = bool(has_int4 and v_format == "mixed")
-    dense_heads = int(cert["dense"].sum())
+    dense_heads = sum(col("dense"))
     stats: dict[str, Any] = {
         "total_blocks": total_blocks, "skipped_blocks": skipped,
         "skip_rate": float(skipped) / float(total_blocks), "attended_blocks": total_blocks - skipped,
@@ -876,54 +898,55 @@ def _assemble_stats(cache, ws: _Workspace, H, G, nq, nact, *, has_int4, force_tr
     stats["rung3_fired"] = bool(dense_heads > 0)
     stats["rung4_fired"] = False
     if has_int4:
-        rho = ws.mass_frac[:, :nq].sum(dim=1)
-        rho_max = float(rho.max().item())
-        eta_int4 = float(cache.values_int4_errors.max().item())
+        rho = tele_f[H: 2 * H].tolist()
+        rho_max = max(rho)
+        eta_int4 = max(tele_f[2 * H: 2 * H + KV].tolist())
         stats["rho_max"] = rho_max
-        stats["rho_mean"] = float(rho.mean().item())
+        stats["rho_mean"] = mean(rho)
         stats["eta_int4"] = eta_int4
         stats["int4_error_bound_loose"] = eta_int4 * rho_max
         stats["int4_error_bound"] = stats["int4_error_bound_loose"]
-        stats["e_val_max"] = float(cert["e_val"].max())
-        stats["e_val_mean"] = float(cert["e_val"].mean())
+        e_val, e_pre = col("e_val"), col("e_pre")
+        stats["e_val_max"] = max(e_val)
+        stats["e_val_mean"] = mean(e_val)
         stats["value_error_mode"] = value_error_mode
-        stats["e_val_pre_rung2_max"] = float(cert["e_pre"].max())
-        stats["e_val_pre_rung2_mean"] = float(cert["e_pre"].mean())
+        stats["e_val_pre_rung2_max"] = max(e_pre)
+        stats["e_val_pre_rung2_mean"] = mean(e_pre)
         if head_blocks:
             stats["value_fallback_blocks"] = union_blocks
             stats["value_fallback_head_blocks"] = head_blocks
-    ks = cert["k_star"]
-    stats["k_star_mean"] = float(ks.astype(np.float32).mean())
-    stats["k_star_min"] = int(ks.min())
-    stats["k_star_max"] = int(ks.max())
+    ks, tail = col("k_star"), col("tail_mass")
+    stats["k_star_mean"] = mean(ks)
+    stats["k_star_min"] = min(ks)
+    stats["k_star_max"] = max(ks)
     stats["tau_cov"] = float(tau_cov) if tau_cov is not None else 0.0
-    stats["tau_cov_actual_mean"] = float(cert["tau_actual"].mean())
-    stats["tail_mass_int8_est_mean"] = float(cert["tail_mass"].mean())
-    stats["tail_mass_int8_est_max"] = float(cert["tail_mass"].max())
+    stats["tau_cov_actual_mean"] = mean(col("tau_actual"))
+    stats["tail_mass_int8_est_mean"] = mean(tail)
+    stats["tail_mass_int8_est_max"] = max(tail)
     stats["rung1_triggered_heads"] = rung1_heads
     stats["rung1_threshold"] = float(rung1_threshold) if rung1_threshold is not None else -1.0
     stats["rung1_multiplier"] = float(rung1_multiplier)
     stats["exploration_rate"] = float(exploration_rate)
-    stats["exploration_blocks"] = int(cert["exploration_blocks"].sum())
-    v_max_layer = cache.v_max_global()
-    stats["v_max_layer"] = float(v_max_layer)
+    stats["exploration_blocks"] = sum(col("exploration_blocks"))
+    v_max_layer = max(tele_f[2 * H + KV: 2 * H + 2 * KV].tolist())
+    stats["v_max_layer"] = v_max_layer
     have_delta = (ranking_fallback or score_consistency_check) and nq > 0
     if have_delta and v_max_layer > 0.0:
-        e2d = np.exp(2.0 * cert["delta"].astype(np.float32))
-        e_key = 2.0 * v_max_layer * e2d * cert["tail_mass"].astype(np.float32) * (e2d - 1.0)
+        e2d = np.exp(2.0 * arr["delta"])
+        e_key = 2.0 * v_max_layer * e2d * arr["tail_mass"] * (e2d - 1.0)
         stats["e_key_step_mean"] = float(e_key.mean())
         stats["e_key_step_max"] = float(e_key.max())
     if score_consistency_check:
         stats["score_consistency_violation_heads"] = violation_heads
-        stats["delta_bound_mean"] = float(cert["delta"].mean())
+        stats["delta_bound_mean"] = mean(delta)
         stats["eps_guard"] = float(eps_guard)
         stats["rung4_fired"] = False
         stats["rung4_violating_heads"] = 0
     if ranking_fallback:
         rk = min(max(int(ranking_r), int(top_k_fp16_keys or 0), 4), nq)
         stats["ranking_heads_total"] = H
-        stats["ranking_disagree_r1"] = int(cert["ranking_disagree_r1"].sum())
-        stats["ranking_disagree_r3"] = int(cert["ranking_disagree_r3"].sum())
+        stats["ranking_disagree_r1"] = sum(col("ranking_disagree_r1"))
+        stats["ranking_disagree_r3"] = sum(col("ranking_disagree_r3"))
         stats["ranking_fallback_triggered"] = dense_heads
         stats["ranking_r"] = int(ranking_r)
         stats["ranking_k"] = int(rk)
@@ -931,11 +954,11 @@ def _assemble_stats(cache, ws: _Workspace, H, G, nq, nact, *, has_int4, force_tr
         stats["boundary_check_triggered_heads"] = boundary_heads
         stats["boundary_check_fired"] = bool(boundary_heads > 0)
         if rk >= 2:
-            gap = (cert["fp16_top1"] - cert["fp16_top2"]).astype(np.float32)
-            stats["score_gap_top12_mean"] = float(gap.mean())
-            stats["score_gap_top12_min"] = float(gap.min())
-        stats["s_int8_top1_mean"] = float(cert["int8_top1"].mean())
-        stats["s_fp16_top1_mean"] = float(cert["fp16_top1"].mean())
+            gap = (arr["fp16_top1"] - arr["fp16_top2"]).tolist()
+            stats["score_gap_top12_mean"] = mean(gap)
+            stats["score_gap_top12_min"] = min(gap)
+        stats["s_int8_top1_mean"] = mean(col("int8_top1"))
+        stats["s_fp16_top1_mean"] = mean(col("fp16_top1"))
     return stats
 
 

@@ -264,6 +264,13 @@ typedef struct {
 } cqa_prefill_item;
 int cqa_prefill_encode(const cqa_prefill_item *items, int n_items, int src_dtype, void *stream);
 
+/* Telemetry of the step whose masks and mass fractions are in `ws`, for hosts that assemble statistics: `out` takes
+ * 2 * H + 2 * KV + CQA_STATS_PARTS 4-byte words: [H] int32 blocks outside the FP16-key mask, [H] float32 sums of the
+ * mass fractions, [KV] float32 largest eta_b, [KV] float32 largest nu_b of the active blocks, [CQA_STATS_PARTS] int32
+ * counts (to be added up) of blocks that at least one head reads from the Tier-2 values. */
+#define CQA_STATS_PARTS 16
+int cqa_step_stats(const cqa_cache *c, const cqa_workspace *ws, int64_t nq, int64_t nact, void *out, void *stream);
+
 /* Fused append-and-quantise of one token at position `pos` for every KV head:
  * Tier-2 rows, nu_b, per-token INT4 (unless `defer_int4`), and, when the token
  * completes a block, the block's INT8 keys and (deferred) INT4 values with
