@@ -56,7 +56,8 @@ int selcert_batched_launch(const cqa_batch_item *items_dev, int n_items, int n_h
                            int q_dtype, int do_append, cudaStream_t st);
 int attend_batched_launch(const cqa_batch_item *items_dev, int n_items, int kv_heads, int gqa_group, int t2_dtype,
                           int max_splits, int q_dtype, float q_scale, int do_append, cudaStream_t st);
-int append_batched_launch(const cqa_batch_item *items_dev, int n_items, int kv_heads, int t2_dtype, int src_dtype, cudaStream_t st);
+int append_batched_launch(const cqa_batch_item *items, cqa_batch_item *dev, int n_items, int kv_heads, int t2_dtype, int src_dtype,
+                          cudaStream_t st);
 int attend_static_launch(const cqa_cache *c, const cqa_workspace *ws, const void *q, int q_dtype, long nq, long nact,
                          long num_tokens, int last_valid, float q_scale, cudaStream_t st);
 
@@ -412,14 +413,15 @@ extern "C" int cqa_layer_step_batched(const cqa_batch_item *items, int n_items, 
         if (it.ws.num_splits > max_splits) max_splits = it.ws.num_splits;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    const cqa_batch_item *dev = static_cast<const cqa_batch_item *>(items_dev);
-    int rc = check_cuda(cudaMemcpyAsync(items_dev, items, (size_t)n_items * sizeof(cqa_batch_item), cudaMemcpyHostToDevice, st),
-                        "copy of the batch records");
-    if (rc) return rc;
+    cqa_batch_item *dev = static_cast<cqa_batch_item *>(items_dev);
+    int rc;
     if (do_append) {
-        rc = append_batched_launch(dev, n_items, c0.kv_heads, c0.t2_dtype, dtype, st);
-        if (rc) return rc;
+        rc = append_batched_launch(items, dev, n_items, c0.kv_heads, c0.t2_dtype, dtype, st);
+    } else {
+        rc = check_cuda(cudaMemcpyAsync(items_dev, items, (size_t)n_items * sizeof(cqa_batch_item), cudaMemcpyHostToDevice, st),
+                        "copy of the batch records");
     }
+    if (rc) return rc;
     rc = score_blocks_batched_launch(dev, n_items, c0.kv_heads, c0.gqa_group, max_nq, dtype, knobs->q_scale, do_append, st);
     if (rc) return rc;
     rc = selcert_batched_launch(dev, n_items, c0.kv_heads * c0.gqa_group, max_nq, knobs, dtype, do_append, st);

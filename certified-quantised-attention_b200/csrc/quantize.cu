@@ -5,6 +5,7 @@
 // owns channel c over the 16 tokens.  Values: thread (t, g) owns group g of
 // token t (16 channels).  All arithmetic that lands in stored bytes is
 // elementwise IEEE; the error norms use the canonical 16-lane dot order.
+#include <cstring>
 #include <type_traits>
 
 #include "common.cuh"
@@ -853,13 +854,65 @@ __global__ void __launch_bounds__(128) append_token_batched_kernel(const cqa_bat
     append_token_body<T2>(it.cache, it.k_new, it.v_new, src_dtype, it.pos, it.defer_int4);
 }
 
-int append_batched_launch(const cqa_batch_item *items_dev, int n_items, int kv_heads, int t2_dtype, int src_dtype, cudaStream_t st)
+// The same with the records as kernel parameters: the CTAs of KV head 0 write them to `dev`, where the other kernels
+// of the step read them.  A copy of the records between two steps cost a transfer through the copy engine in the
+// middle of a chain of kernels.
+template <int N>
+struct BatchRecords {
+    cqa_batch_item it[N];
+};
+constexpr int RECORDS_SMALL = 8, RECORDS_LARGE = 40;
+static_assert(sizeof(BatchRecords<RECORDS_LARGE>) + 16 <= 32764, "limit of a kernel's parameters");
+template <typename T2, int N>
+__global__ void __launch_bounds__(128) append_token_records_kernel(const __grid_constant__ BatchRecords<N> rec, cqa_batch_item *dev, int src_dtype)
 {
-    dim3 grid((unsigned)kv_heads, (unsigned)n_items);
+    grid_dependency_wait();          // the previous step's kernels have read their records
+    const cqa_batch_item &it = rec.it[blockIdx.y];
+    if (blockIdx.x == 0) {
+        const int *from = reinterpret_cast<const int *>(&it);
+        int *to = reinterpret_cast<int *>(dev + blockIdx.y);
+        for (int i = threadIdx.x; i < (int)(sizeof(cqa_batch_item) / 4); i += blockDim.x) to[i] = from[i];
+    }
+    append_token_body<T2>(it.cache, it.k_new, it.v_new, src_dtype, it.pos, it.defer_int4);
+}
+
+template <typename T2, int N>
+static int append_records_n(const cqa_batch_item *items, cqa_batch_item *dev, int n_items, int kv_heads, int src_dtype, cudaStream_t st)
+{
+    BatchRecords<N> rec;
+    memcpy(rec.it, items, (size_t)n_items * sizeof(cqa_batch_item));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)kv_heads, (unsigned)n_items);
+    cfg.blockDim = dim3(128);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    void *args[] = {&rec, &dev, &src_dtype};
+    note_launch();
+    return check_cuda(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void *>(append_token_records_kernel<T2, N>), args), "append_token_records_kernel");
+}
+template <typename T2>
+static int append_batched_t(const cqa_batch_item *items, cqa_batch_item *dev, int n_items, int kv_heads, int src_dtype, cudaStream_t st)
+{
+    if (n_items <= RECORDS_SMALL) return append_records_n<T2, RECORDS_SMALL>(items, dev, n_items, kv_heads, src_dtype, st);
+    if (n_items <= RECORDS_LARGE) return append_records_n<T2, RECORDS_LARGE>(items, dev, n_items, kv_heads, src_dtype, st);
+    int rc = check_cuda(cudaMemcpyAsync(dev, items, (size_t)n_items * sizeof(cqa_batch_item), cudaMemcpyHostToDevice, st),
+                        "copy of the batch records");
+    if (rc) return rc;
+    return check_cuda(launch_chained(append_token_batched_kernel<T2>, dim3((unsigned)kv_heads, (unsigned)n_items), dim3(128), 0, st, true,
+                                     dev, src_dtype), "append_token_batched_kernel");
+}
+
+// Appends the batch's tokens and leaves the records on the device.
+int append_batched_launch(const cqa_batch_item *items, cqa_batch_item *dev, int n_items, int kv_heads, int t2_dtype, int src_dtype, cudaStream_t st)
+{
     switch (t2_dtype) {
-    case CQA_F32: return check_cuda(launch_chained(append_token_batched_kernel<float>, grid, dim3(128), 0, st, true, items_dev, src_dtype), "append_token_batched_kernel");
-    case CQA_F16: return check_cuda(launch_chained(append_token_batched_kernel<__half>, grid, dim3(128), 0, st, true, items_dev, src_dtype), "append_token_batched_kernel");
-    default: return check_cuda(launch_chained(append_token_batched_kernel<__nv_bfloat16>, grid, dim3(128), 0, st, true, items_dev, src_dtype), "append_token_batched_kernel");
+    case CQA_F32: return append_batched_t<float>(items, dev, n_items, kv_heads, src_dtype, st);
+    case CQA_F16: return append_batched_t<__half>(items, dev, n_items, kv_heads, src_dtype, st);
+    default: return append_batched_t<__nv_bfloat16>(items, dev, n_items, kv_heads, src_dtype, st);
     }
 }
 

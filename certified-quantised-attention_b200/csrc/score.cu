@@ -228,6 +228,7 @@ template <int G>
 __global__ void __launch_bounds__(SCORE_WARPS * 32, 2) score_blocks_batched_kernel(const cqa_batch_item *items, int q_dtype,
                                                                                   float q_scale, int do_append)
 {
+    grid_dependency_wait();      // the append kernel may be what writes the records
     const cqa_batch_item &it = *stage_batch_item(items + blockIdx.z);
     const long nq = (it.pos + do_append) / BS;
     long bpc = (nq + gridDim.x - 1) / gridDim.x;

@@ -16,7 +16,9 @@ when `collect_stats` is set.  There is no Triton, PyTorch or CPU compute path.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
+import weakref
 from typing import Any
 
 import numpy as np
@@ -36,6 +38,7 @@ DEFAULT_RUNG1_MULTIPLIER = 2.0
 _CERT_INT_FIELDS = [f for f, t in _lib.CqaHeadCert._fields_ if t is C.c_int32]
 _CERT_F32_FIELDS = [f for f, t in _lib.CqaHeadCert._fields_ if t is C.c_float]
 _CERT_DTYPE = np.dtype(_lib.CqaHeadCert)
+_BATCH_DTYPE = np.dtype(_lib.CqaBatchItem)
 
 
 # ----------------------------------------------------------------------------- workspace
@@ -228,6 +231,7 @@ def _make_knobs(*, q_scale, tau_cov, k_min, k_max, rung1_threshold, rung1_multip
     return k
 
 
+@functools.lru_cache(maxsize=4096)
 def _selection_width(k_max, rung1_threshold, rung1_multiplier, nq: int) -> int:
     if k_max is None:
         return nq
@@ -457,6 +461,7 @@ def certified_decode_token_host(
     return out_host
 
 
+@functools.lru_cache(maxsize=4096)
 def _batch_splits(slots: int, heads: int, nact: int, limit: int) -> int:
     """Phase-2 splits per (sequence, KV head) of a batch: the count that minimises (waves of `slots` resident CTAs)
     x (blocks per CTA + the fixed cost of a CTA, worth about 64 blocks: merges, partial rows, ticket).  Rounding the
@@ -537,63 +542,106 @@ def certified_attention_batch(
         score_consistency_check=score_consistency_check, value_error_mode=value_error_mode,
         force_trailing_value_fp16=True,
     )
-    key = (tuple(id(c) for c in caches), G)
     plan = getattr(first, "_batch_plan", None)
-    if plan is None or plan[0] != key:
-        items = (_lib.CqaBatchItem * B)()
-        items_dev = torch.empty(C.sizeof(items) + 16, dtype=torch.uint8, device=device)
-        out = torch.empty(B, H, first.head_dim, dtype=torch.float32, device=device)
-        plan = (key, items, items_dev, out)
-        first._batch_plan = plan
-    _, items, items_dev, out = plan
-    esz = q.element_size()
-    row_q, row_kv = H * first.head_dim * esz, KV * first.head_dim * esz
+    if plan is None or not plan.current(caches, G):
+        plan = first._batch_plan = _BatchPlan(caches, G, device)
+    positions = [c.num_tokens for c in caches]
+    pos = np.array(positions, dtype=np.int64)
+    n_tok = pos + (1 if do_append else 0)
     block = first.block_size
-    sms = torch.cuda.get_device_properties(device).multi_processor_count
-    positions = []
-    for b, cache in enumerate(caches):
-        if (cache.kv_heads, cache.head_dim, cache.keys_int8.device) != (KV, first.head_dim, first.keys_int8.device):
-            raise ValueError("all caches of a batch must share geometry and device")
-        pos = cache.num_tokens
-        if do_append and pos >= cache.keys_int8.shape[1]:
-            raise ValueError(f"cache capacity {cache.keys_int8.shape[1]} exhausted")
-        n_tok = pos + (1 if do_append else 0)
-        nq, nact = n_tok // block, (n_tok + block - 1) // block
-        if nq <= 0:
-            raise NotImplementedError("the certified path needs at least one complete block per sequence")
-        ws = _workspace(cache, H, G, device)
-        ws.ensure_sel_width(_selection_width(k_max, rung1_threshold, rung1_multiplier, nq), device)
-        w = ws.fill_struct(nact)
-        # splits per sequence: never more than the sequence's own limit (its partial buffers)
-        ns = int(num_splits) if num_splits else _batch_splits(2 * sms, KV * B, nact, w.num_splits)
-        w.num_splits = max(1, min(ns, w.num_splits, nact))
-        if exploration_rate > 0.0:
-            w.rng_seed = ws.draw_seed()
-            w.rng_offset = ws.rng_calls
+    nq, nact = n_tok // block, (n_tok + block - 1) // block
+    if do_append and (pos >= plan.caps).any():
+        raise ValueError(f"cache capacity {int(plan.caps[pos >= plan.caps][0])} exhausted")
+    if int(nq.min()) <= 0:
+        raise NotImplementedError("the certified path needs at least one complete block per sequence")
+    # the widths follow the lengths; a workspace that has to grow makes the records stale
+    widths = [_selection_width(k_max, rung1_threshold, rung1_multiplier, n) for n in nq.tolist()]
+    if any(w > have for w, have in zip(widths, plan.sel_widths)):
+        for (_, ws), w in zip(plan.refs, widths):
+            ws().ensure_sel_width(w, device)
+        plan = first._batch_plan = _BatchPlan(caches, G, device)
+    # Phase-2 splits per sequence: never more than the sequence's own limit (its partial buffers)
+    ns, ds = [], []
+    for n, own, dense in zip(nact.tolist(), plan.num_splits, plan.dense_splits):
+        limit = max(1, min(own, (n + 7) // 8))
+        want = int(num_splits) if num_splits else _batch_splits(2 * plan.sms, KV * B, n, limit)
+        ns.append(max(1, min(want, limit, n)))
+        ds.append(max(1, min(dense, (n + 15) // 16)))
+    rec = plan.records
+    rec["pos"] = pos
+    rec["ws"]["num_splits"] = ns
+    rec["ws"]["dense_splits"] = ds
+    esz = q.element_size()
+    order = plan.order
+    rec["q"] = q.data_ptr() + order * (H * first.head_dim * esz)
+    if do_append:
+        row_kv = KV * first.head_dim * esz
+        rec["k_new"] = new_keys.data_ptr() + order * row_kv
+        rec["v_new"] = new_values.data_ptr() + order * row_kv
+    else:
+        rec["k_new"] = 0
+        rec["v_new"] = 0
+    rec["defer_int4"] = [1 if c._defers_int4() else 0 for c in caches]
+    if exploration_rate > 0.0:
+        spaces = [ws() for _, ws in plan.refs]
+        rec["ws"]["rng_seed"] = np.array([ws.draw_seed() for ws in spaces], dtype=np.uint64)
+        rec["ws"]["rng_offset"] = [ws.rng_calls for ws in spaces]
+        for ws in spaces:
             ws.rng_calls += 1
-        it = items[b]
-        C.memmove(C.byref(it.cache), C.byref(cache._desc(G)), C.sizeof(_lib.CqaCache))
-        C.memmove(C.byref(it.ws), C.byref(w), C.sizeof(_lib.CqaWorkspace))
-        it.ws.out = out.data_ptr() + b * H * first.head_dim * 4
-        it.q = q.data_ptr() + b * row_q
-        it.k_new = new_keys.data_ptr() + b * row_kv if do_append else None
-        it.v_new = new_values.data_ptr() + b * row_kv if do_append else None
-        it.pos = pos
-        it.defer_int4 = 1 if cache._defers_int4() else 0
-        positions.append(pos)
-    dev_ptr = (items_dev.data_ptr() + 15) & ~15
     stream = _lib.current_stream(device)
     with _lib.on_device(device):
-        _lib.check(_lib.lib().cqa_layer_step_batched(items, B, dev_ptr, C.byref(knobs), _lib.dtype_code(q.dtype),
+        _lib.check(_lib.lib().cqa_layer_step_batched(plan.items, B, plan.dev_ptr, C.byref(knobs), _lib.dtype_code(q.dtype),
                                                      1 if do_append else 0, stream), "cqa_layer_step_batched")
-        for b, cache in enumerate(caches):
-            if cache.bounded_hot_tier:
-                n_tok = positions[b] + (1 if do_append else 0)
-                cache._hot_tier_update(cache._desc(G), items[b].ws, (n_tok + block - 1) // block, stream)
+        for b in plan.bounded:
+            caches[b]._hot_tier_update(caches[b]._desc(G), plan.items[b].ws, int(nact[b]), stream)
     if do_append:
-        for b, cache in enumerate(caches):
-            cache._advance_after_append(positions[b])
-    return out
+        for cache, p in zip(caches, positions):
+            cache._advance_after_append(p)
+    return plan.out
+
+
+class _BatchPlan:
+    """The records of one batch of caches, kept on its first cache.  What depends on the buffers only is written here;
+    per call the position, split counts and row pointers of all sequences are written as columns."""
+
+    def __init__(self, caches, G: int, device):
+        first, B = caches[0], len(caches)
+        H = first.kv_heads * G
+        for cache in caches:
+            if (cache.kv_heads, cache.head_dim, cache.keys_int8.device) != (first.kv_heads, first.head_dim, first.keys_int8.device):
+                raise ValueError("all caches of a batch must share geometry and device")
+        self.G = G
+        spaces = [_workspace(c, H, G, device) for c in caches]
+        self.refs = [(weakref.ref(c), weakref.ref(w)) for c, w in zip(caches, spaces)]   # the plan keeps no cache alive
+        self.descs = [c._desc(G) for c in caches]
+        self.items = (_lib.CqaBatchItem * B)()
+        self.records = np.frombuffer(self.items, dtype=_BATCH_DTYPE)
+        self.order = np.arange(B, dtype=np.uint64)
+        items_dev = torch.empty(C.sizeof(self.items) + 16, dtype=torch.uint8, device=device)
+        self.items_dev = items_dev
+        self.dev_ptr = (items_dev.data_ptr() + 15) & ~15
+        self.out = torch.empty(B, H, first.head_dim, dtype=torch.float32, device=device)
+        self.caps = np.array([c.keys_int8.shape[1] for c in caches], dtype=np.int64)
+        self.bounded = [b for b, c in enumerate(caches) if c.bounded_hot_tier]
+        self.sms = torch.cuda.get_device_properties(device).multi_processor_count
+        for b, (ws, desc) in enumerate(zip(spaces, self.descs)):
+            C.memmove(C.byref(self.items[b].cache), C.byref(desc), C.sizeof(_lib.CqaCache))
+            C.memmove(C.byref(self.items[b].ws), C.byref(ws.fill_struct()), C.sizeof(_lib.CqaWorkspace))
+            self.items[b].ws.out = self.out.data_ptr() + b * H * first.head_dim * 4
+        self.sel_widths = [ws.sel_width for ws in spaces]
+        self.num_splits = [ws.num_splits for ws in spaces]
+        self.dense_splits = [ws.dense_splits for ws in spaces]
+
+    def current(self, caches, G: int) -> bool:
+        """Whether the records still describe these caches, their workspaces and descriptors."""
+        if G != self.G or len(caches) != len(self.refs):
+            return False
+        for cache, (mine, space), desc, ns, ds in zip(caches, self.refs, self.descs, self.num_splits, self.dense_splits):
+            ws = cache._certified_workspace.get("cqa_ws")
+            if (cache is not mine() or ws is None or ws is not space() or ws._struct_stale
+                    or cache._desc_cache.get(G) is not desc or ws.num_splits != ns or ws.dense_splits != ds):
+                return False
+        return True
 
 
 def certified_attention_layer(
