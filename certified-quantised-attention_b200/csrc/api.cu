@@ -436,9 +436,7 @@ extern "C" int cqa_suggest_splits(int kv_heads, int gqa_group, int64_t nact, int
         set_error("cqa_suggest_splits: bad arguments");
         return CQA_ERR_INVALID;
     }
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
+    const int sms = sm_count();
     // Phase 2: two resident CTAs per SM, at least 8 blocks (one per warp) per split.
     long target = ((long)sms * CQA_ATT_MIN_CTAS) / kv_heads;
     if (target < 1) target = 1;
@@ -447,8 +445,8 @@ extern "C" int cqa_suggest_splits(int kv_heads, int gqa_group, int64_t nact, int
     if (ns > CQA_MAX_SPLITS) ns = CQA_MAX_SPLITS;
     if (ns < 1) ns = 1;
     *num_splits = (int)ns;
-    // dense recompute: chunks of about 16 blocks per (flagged head), at most CQA_MAX_DENSE_SPLITS
-    long ds = (nact + 15) / 16;
+    // dense recompute: chunks of about 8 blocks (one per warp) per flagged head, at most CQA_MAX_DENSE_SPLITS
+    long ds = (nact + 7) / 8;
     if (ds > CQA_MAX_DENSE_SPLITS) ds = CQA_MAX_DENSE_SPLITS;
     if (ds < 1) ds = 1;
     *dense_splits = (int)ds;

@@ -9,7 +9,8 @@
 //   * (head, block) pairs flagged in topk_mask take their logits from Tier-2 keys, pairs flagged in value_mask their
 //     values from Tier 2: the same products, the four heads together.  The rows are requested into L2 two pairs ahead.
 //   * Heads that the certificate flags for the dense FP16 recompute: when a CTA is done with its split it takes units
-//     of (group with a flagged head, chunk of blocks).  With no flagged head this is one word read.
+//     of (group with a flagged head, chunk of blocks); CTAs beyond the splits, where the GPU has room for them, start
+//     there.  With no flagged head this is one word read.
 //   * The last CTA to finish for a KV head (a group, for the dense part) merges the split partials and writes the
 //     output rows; no separate merge launch.
 //
@@ -158,7 +159,7 @@ struct AttLayout {
     // cross-warp merge buffers and final-merge scratch (both alias the ring)
     static constexpr int MERGE_A = ATT_WARPS * HG * (D + 2) * 4;
     static constexpr int MERGE_B = (2 * G * CQA_MAX_SPLITS + G + 4 + ATT_WARPS * D) * 4;
-    static constexpr int MERGE_D = (2 * CQA_MAX_DENSE_SPLITS + 8 + ATT_WARPS * D) * 4;
+    static constexpr int MERGE_D = (2 * HG * CQA_MAX_DENSE_SPLITS + HG + 4 + ATT_WARPS * D) * 4;
     static constexpr int MERGE = MERGE_A > MERGE_B ? (MERGE_A > MERGE_D ? MERGE_A : MERGE_D) : (MERGE_B > MERGE_D ? MERGE_B : MERGE_D);
     static constexpr int RING_BYTES = RING > MERGE ? RING : MERGE;
     // the query as matrix fragments: [pieces 0,1 | piece 2][8 steps][32 lanes] words of two 16-bit pairs; with float32
@@ -290,14 +291,22 @@ struct AttWarp {
                     if (!(km & (1u << g))) continue;
                     float qv[8];
                     load8<float>(qrow + g * D + 8 * L, qv);
+                    float p[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const int t = hw * 8 + half * 4 + i;
                         float kf[8];
                         raw_to_f(kr[i], kf);
-                        const float d = hw_sum(chain8(kf, qv));
-                        if (L == 0) sc[g * BS + t] = t < n_valid ? d * q_scale : -INFINITY;
+                        p[i] = chain8(kf, qv);
                     }
+                    // sums over the 16 lanes of four rows at once: lane L ends with row i = L / 4
+                    const bool u8 = (L & 8) != 0, u4 = (L & 4) != 0;
+                    const float a0 = (u8 ? p[2] : p[0]) + __shfl_xor_sync(FULL, u8 ? p[0] : p[2], 8);
+                    const float a1 = (u8 ? p[3] : p[1]) + __shfl_xor_sync(FULL, u8 ? p[1] : p[3], 8);
+                    float d = (u4 ? a1 : a0) + __shfl_xor_sync(FULL, u4 ? a0 : a1, 4);
+                    d += __shfl_xor_sync(FULL, d, 2);
+                    d += __shfl_xor_sync(FULL, d, 1);
+                    const int t = hw * 8 + half * 4 + (L >> 2);
+                    if ((L & 3) == 0) sc[g * BS + t] = t < n_valid ? d * q_scale : -INFINITY;
                 }
             }
         } else {
@@ -600,7 +609,8 @@ __device__ __forceinline__ void cta_merge_store(const float *sm_m, const float *
 // one warp per head turns them into per-split scales while those loads are still travelling; the rows are then
 // scaled and summed, the per-thread sums combined through shared memory, normalised and written.
 __device__ __forceinline__ void final_merge(const float *pm, const float *pl, const float *pa, int ns, int head0,
-                                            int nh, const cqa_workspace &ws, bool dense_role, float *sm, int kv_heads, int n_heads_total)
+                                            int nh, const cqa_workspace &ws, bool dense_role, float *sm, int kv_heads, int n_heads_total,
+                                            int arrivals = 1)
 {
     constexpr int BATCH = 20;
     const bool push_c = ws.partial_out != nullptr && ws.peer_world > 0 && ws.peer_partial[0] != nullptr;
@@ -702,8 +712,8 @@ __device__ __forceinline__ void final_merge(const float *pm, const float *pl, co
         __threadfence_system();
         int expected = kv_heads;
         if (ws.dense_splits > 0 && ws.cert != nullptr) expected += ws.any_flags[2] ? n_heads_total : ws.any_flags[4];
-        const int t = atomicAdd(ws.peer_ticket_c, 1);
-        if (t == expected - 1) {
+        const int t = atomicAdd(ws.peer_ticket_c, arrivals);
+        if (t == expected - arrivals) {
             *ws.peer_ticket_c = 0;
             __threadfence_system();
             for (int p = 0; p < ws.peer_world; ++p)
@@ -751,7 +761,7 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
     const int ns = ws.num_splits, split = (int)blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b_begin = split * blocks_per_split;
-    const int b_end = ns > 0 ? min((int)nact, b_begin + blocks_per_split) : b_begin;
+    const int b_end = split < ns ? min((int)nact, b_begin + blocks_per_split) : b_begin;      // CTAs x >= ns: dense recompute only
     const int my_first = b_begin + 2 * warp;     // this warp's blocks: pairs my_first + 16 * it
     char *ring = dsm, *wring = ring + warp * ATT_STAGES * LY::STAGE;
     char *qfrag = dsm + LY::RING_BYTES;
@@ -948,7 +958,7 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
     float *sm_m = reinterpret_cast<float *>(ring);
     float *sm_l = sm_m + ATT_WARPS * HG;
     float *sm_acc = sm_l + ATT_WARPS * HG;
-    if (ns > 0) {
+    if (split < ns) {
         __syncthreads();  // the ring is reused as merge buffers
         W.store(sm_m, sm_l, sm_acc, warp);
         cta_merge_store<HG>(sm_m, sm_l, sm_acc, ws.part_m, ws.part_l, ws.part_acc, head0, split, ns);
@@ -958,33 +968,50 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
     }
     if (n_dense == 0) return;
 
-    // ---- dense recompute of the flagged heads: units of (group of heads with a flagged one, chunk of blocks) over all
-    // CTAs; the heads of a group share the rows.
-    const int groups = c.kv_heads * SUBS, ds = ws.dense_splits;
-    const int n_ctas = (ns > 0 ? ns : (int)gridDim.x) * groups;
-    const int id = (int)blockIdx.y * (ns > 0 ? ns : (int)gridDim.x) + split;
+    // ---- dense recompute of the flagged heads: units of (group of heads with a flagged one, chunk of blocks), dealt to
+    // the CTAs without a split first; the heads of a group share the rows.
+    constexpr int WINDOW = 256;          // groups looked at together
+    __shared__ unsigned char s_group[WINDOW], s_heads[WINDOW];
+    __shared__ int s_count;
+    const int groups = c.kv_heads * SUBS, ds = ws.dense_splits, gx = (int)gridDim.x, spare = gx - ns;
+    const int n_ctas = gx * groups;
+    const int id = (split >= ns ? split - ns : spare + split) * groups + (int)blockIdx.y;
     const long nblk = (num_tokens + BS - 1) / BS, bps = (nblk + ds - 1) / ds;
-    int loaded = (int)blockIdx.y, unit0 = 0;
+    int loaded = (int)blockIdx.y;
 #pragma unroll 1
-    for (int y = 0; y < groups; ++y) {
-        const int dkv = y / SUBS, dh0 = dkv * G + (y % SUBS) * HG;
-        const int f = lane < HG ? (dense_all || ws.cert[dh0 + lane].dense) : 0;
-        const unsigned heads = __ballot_sync(FULL, f != 0);
-        if (heads == 0) continue;
-        const int first = unit0;
-        unit0 += ds;
-        // this CTA's chunks of the group: units u = id, id + n_ctas, ... within [first, first + ds)
-        int u = id + ((first - id + n_ctas - 1) / n_ctas) * n_ctas;
-        if (id >= first) u = id;
+    for (int g0 = 0; g0 < groups; g0 += WINDOW) {
+        const int in_window = min(groups - g0, WINDOW);
+        __syncthreads();
+        if ((int)threadIdx.x < in_window) {
+            unsigned heads = 0;
+            const int y = g0 + (int)threadIdx.x, dh0 = (y / SUBS) * G + (y % SUBS) * HG;
+#pragma unroll
+            for (int g = 0; g < HG; ++g) heads |= (dense_all || ws.cert[dh0 + g].dense) ? 1u << g : 0u;
+            s_heads[threadIdx.x] = (unsigned char)heads;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            int n = 0;
+            for (int i = 0; i < in_window; i += 32) {
+                const bool f = i + lane < in_window && s_heads[i + lane] != 0;
+                const unsigned who = __ballot_sync(FULL, f);
+                if (f) s_group[n + __popc(who & ((1u << lane) - 1u))] = (unsigned char)(i + lane);
+                n += __popc(who);
+            }
+            if (lane == 0) s_count = n;
+        }
+        __syncthreads();
+        const int n_groups = s_count;
 #pragma unroll 1
-        for (; u < first + ds; u += n_ctas) {
-            const int chunk = u - first;
+        for (int u = id; u < n_groups * ds; u += n_ctas) {
+            const int at = s_group[u % n_groups], chunk = u / n_groups, y = g0 + at;
+            const unsigned heads = s_heads[at];
+            const int dkv = y / SUBS, dh0 = dkv * G + (y % SUBS) * HG;
             if (loaded != y) {
                 __syncthreads();
                 third = load_query(dh0);
                 loaded = y;
             }
-            __syncthreads();      // the ring was merge scratch
             const long d0 = (long)chunk * bps, d1 = min(nblk, d0 + bps);
             W.init(lane, -INFINITY, 32768.0f);
             float *sc = reinterpret_cast<float *>(wring + LY::SCORES);
@@ -1007,12 +1034,10 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
             __syncthreads();
             W.store(sm_m, sm_l, sm_acc, warp);
             cta_merge_store<HG>(sm_m, sm_l, sm_acc, ws.dense_m, ws.dense_l, ws.dense_acc, dh0, chunk, ds);
-            if (take_ticket(ws.tickets + c.kv_heads + dh0, ds, &s_flag)) {
-                for (int g = 0; g < HG; ++g)
-                    if (heads & (1u << g))
-                        final_merge(ws.dense_m, ws.dense_l, ws.dense_acc, ds, dh0 + g, 1, ws, true, reinterpret_cast<float *>(ring),
-                                    c.kv_heads, c.kv_heads * G);
-            }
+            if (take_ticket(ws.tickets + c.kv_heads + dh0, ds, &s_flag))
+                final_merge(ws.dense_m, ws.dense_l, ws.dense_acc, ds, dh0, HG, ws, true, reinterpret_cast<float *>(ring), c.kv_heads,
+                            c.kv_heads * G, __popc(heads));
+            __syncthreads();      // the ring is merge scratch
         }
     }
 }
@@ -1035,9 +1060,17 @@ __global__ void __launch_bounds__(ATT_THREADS, CQA_ATT_MIN_CTAS) attend_batched_
     const long num_tokens = it.pos + do_append;
     const long nq = num_tokens / BS, nact = (num_tokens + BS - 1) / BS;
     const int ns = it.ws.num_splits;
-    if ((int)blockIdx.x >= ns) return;
     const int last_valid = nact == nq ? BS : (int)(num_tokens - nq * BS);
     attend_body<G, T2>(it.cache, it.ws, it.q, q_dtype, nq, nact, num_tokens, last_valid, q_scale, (int)((nact + ns - 1) / ns));
+}
+
+// Columns of CTAs beside the splits that only take part in the dense recompute: what fits the first wave, at most
+// eight.  A short context leaves most of the GPU idle, and a recompute behind the splits of a few CTAs cost it 8 us;
+// a long one fills the GPU with splits, and the recompute follows on all of them.
+static int spare_columns(int splits, long rows)
+{
+    const long slots = (long)sm_count() * CQA_ATT_MIN_CTAS, left = slots - rows * splits;
+    return (int)(left <= 0 ? 0 : (left / rows < 8 ? left / rows : 8));
 }
 
 template <int G, typename T2>
@@ -1056,7 +1089,8 @@ static int attend_launch_gt(const cqa_cache *c, const cqa_workspace *ws, const v
     static size_t granted[SMEM_ATTR_DEVICES] = {};
     const int rc_attr = check_cuda(ensure_dynamic_smem(attend_kernel<G, T2>, smem, granted), "cudaFuncSetAttribute(attend_kernel)");
     if (rc_attr) return rc_attr;
-    dim3 grid((unsigned)ns, (unsigned)(c->kv_heads * AttLayout<G, T2>::SUBS));
+    const int rows = c->kv_heads * AttLayout<G, T2>::SUBS;
+    dim3 grid((unsigned)(ns + (dense ? spare_columns(ns, rows) : 0)), (unsigned)rows);
     return check_cuda(launch_chained(attend_kernel<G, T2>, grid, dim3(ATT_THREADS), smem, st, chained, *c, w, q, q_dtype, nq,
                                      nact, num_tokens, last_valid, q_scale, bps),
                       "attend_kernel");
@@ -1141,7 +1175,8 @@ static int attend_batched_launch_gt(const cqa_batch_item *items_dev, int n_items
     const int rc = check_cuda(ensure_dynamic_smem(attend_batched_kernel<G, T2>, smem, granted),
                               "cudaFuncSetAttribute(attend_batched_kernel)");
     if (rc) return rc;
-    dim3 grid((unsigned)max_splits, (unsigned)(kv_heads * AttLayout<G, T2>::SUBS), (unsigned)n_items);
+    const int rows = kv_heads * AttLayout<G, T2>::SUBS;
+    dim3 grid((unsigned)(max_splits + spare_columns(max_splits, (long)rows * n_items)), (unsigned)rows, (unsigned)n_items);
     return check_cuda(launch_chained(attend_batched_kernel<G, T2>, grid, dim3(ATT_THREADS), smem, st, true, items_dev, q_dtype,
                                      q_scale, do_append), "attend_batched_kernel");
 }
@@ -1183,7 +1218,7 @@ static int dense_launch_t(const cqa_cache *c, const cqa_workspace *ws, const voi
 #define CQA_DENSE_CASE(GG)                                                                                             \
     case GG: {                                                                                                         \
         const int rows = c->kv_heads * AttLayout<GG, T2>::SUBS;                                                        \
-        dim3 grid((unsigned)((296 + rows - 1) / rows), (unsigned)rows);                                                \
+        dim3 grid((unsigned)((sm_count() * CQA_ATT_MIN_CTAS + rows - 1) / rows), (unsigned)rows);                      \
         const size_t smem = attend_smem<GG, T2>();                                                                         \
         static size_t granted[SMEM_ATTR_DEVICES] = {};                                                                 \
         const int rc = check_cuda(ensure_dynamic_smem(attend_kernel<GG, T2>, smem, granted), "cudaFuncSetAttribute(attend_kernel)"); \

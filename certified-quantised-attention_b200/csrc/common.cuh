@@ -320,6 +320,19 @@ static inline cudaError_t ensure_dynamic_smem(K kernel, size_t bytes, size_t (&g
     return e;
 }
 
+// SMs of the current device (asked once per device).
+static inline int sm_count()
+{
+    static int known[SMEM_ATTR_DEVICES] = {};
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    const bool tracked = dev >= 0 && dev < SMEM_ATTR_DEVICES;
+    if (tracked && known[dev] > 0) return known[dev];
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    if (tracked) known[dev] = n;
+    return n;
+}
+
 // Launch with (or without) the programmatic-serialisation attribute.
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,

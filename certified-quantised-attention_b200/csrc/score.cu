@@ -294,15 +294,11 @@ static int score_launch_g(const cqa_cache *c, const void *q, int q_dtype, long n
 int score_blocks_batched_launch(const cqa_batch_item *items_dev, int n_items, int kv_heads, int gqa_group, long max_nq,
                                 int q_dtype, float q_scale, int do_append, cudaStream_t st)
 {
-    int dev = 0, sm_count = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-    if (sm_count <= 0) sm_count = 148;
     // CTAs per (sequence, KV head): the count that minimises (waves of 2 CTAs per SM) x (blocks per CTA + a fixed
     // start-up cost of about 16 blocks).  One CTA too many per head spills the grid into a second, nearly empty wave
     // (5 instead of 4 CTAs per head cost 9 % of a 128K batch of 8); with many waves the granularity of a
     // one-sequence launch is the best choice again.  The split does not change any result: blocks are independent.
-    const long slots = (long)sm_count * 2, heads = (long)kv_heads * n_items;
+    const long slots = (long)sm_count() * 2, heads = (long)kv_heads * n_items;
     long p_max = (slots + kv_heads - 1) / kv_heads;          // what a launch for one sequence uses
     const long by_work = (max_nq + 15) / 16;                  // at least 16 blocks per CTA
     if (p_max > by_work) p_max = by_work;
@@ -356,15 +352,8 @@ int score_blocks_launch(const cqa_cache *c, const void *q, int q_dtype, long nq,
 {
     ScorePush push = {};
     if (push_in) push = *push_in;
-    static int sm_count = 0;
-    if (sm_count == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-        if (sm_count <= 0) sm_count = 148;
-    }
     // two resident CTAs per SM
-    long target_ctas = (long)sm_count * 2;
+    long target_ctas = (long)sm_count() * 2;
     long per_kv = (target_ctas + c->kv_heads - 1) / c->kv_heads;
     long bpc = (nq + per_kv - 1) / per_kv;
     if (bpc < 2) bpc = 2;

@@ -149,7 +149,7 @@ class _Workspace:
         if nact is not None:
             # never more splits than eight-block groups of work
             ns = max(1, min(ns, (nact + 7) // 8))
-            ds = max(1, min(ds, (nact + 15) // 16))
+            ds = max(1, min(ds, (nact + 7) // 8))
         s.num_splits, s.dense_splits = ns, ds
         return s
 
@@ -566,7 +566,7 @@ def certified_attention_batch(
         limit = max(1, min(own, (n + 7) // 8))
         want = int(num_splits) if num_splits else _batch_splits(2 * plan.sms, KV * B, n, limit)
         ns.append(max(1, min(want, limit, n)))
-        ds.append(max(1, min(dense, (n + 15) // 16)))
+        ds.append(max(1, min(dense, (n + 7) // 8)))
     rec = plan.records
     rec["pos"] = pos
     rec["ws"]["num_splits"] = ns
