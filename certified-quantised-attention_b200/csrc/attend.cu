@@ -170,20 +170,22 @@ struct AttLayout {
     static constexpr int TOTAL = RING_BYTES + QFRAG + ATT_WARPS * WTILE;
 };
 
-// Per-lane source pointers of the next pair of blocks to stage.
+// Per-lane source pointers of the next unit (block or pair of blocks) to stage.
 template <int G, typename T2>
 struct AttIssuer {
     using LY = AttLayout<G, T2>;
     const char *pk, *s, *z, *sc;   // global sources for this lane
-    int b, b_end, nq;              // first block of the pair to issue next
+    int b, b_end;                  // first block of the unit to issue next
+    int unit;                      // blocks of a unit: 1 or 2
     int at;                        // swizzled place of this lane's 16 code bytes within 512
     bool have4;
 
-    __device__ __forceinline__ void init(const cqa_cache &c, const float *tok, int nq_, int kv, int sub, int b0, int bend, int lane)
+    __device__ __forceinline__ void init(const cqa_cache &c, const float *tok, int nq_, int kv, int sub, int b0, int bend, int unit_,
+                                         int lane)
     {
         b = b0;
         b_end = min(bend, nq_);
-        nq = nq_;
+        unit = unit_;
         have4 = c.values_int4_packed != nullptr;
         const int t = lane >> 2;
         at = t * 64 + 16 * ((lane & 3) ^ ((t >> 1) & 3));      // eight tokens per round, the same pattern in each
@@ -195,12 +197,12 @@ struct AttIssuer {
         sc = reinterpret_cast<const char *>(tok + ((long)kv * nq_ + b0 + lane / (4 * LY::HG)) * G * BS + sub * LY::HG * BS) +
              (lane % (4 * LY::HG)) * 16;
     }
-    // Stage blocks b and b + 1 (as far as they are quantised blocks of this CTA) and advance by a warp stride; always
+    // Stage the unit's blocks (as far as they are quantised blocks of this CTA) and advance by a warp stride; always
     // commits one group.
     __device__ __forceinline__ void issue(char *stage, int lane)
     {
         if (b < b_end) {
-            const bool two = b + 1 < b_end;
+            const bool two = unit == 2 && b + 1 < b_end;
             if (have4) {
                 att_cp16(stage + at, pk);
                 att_cp16(stage + at + 512, pk + 512);
@@ -219,11 +221,12 @@ struct AttIssuer {
             }
         }
         att_commit();
-        b += 2 * ATT_WARPS;
-        pk += 2 * ATT_WARPS * BS * (D / 2);
-        s += 2 * ATT_WARPS * BS * NG * 2;
-        z += 2 * ATT_WARPS * BS * NG * 2;
-        sc += 2 * ATT_WARPS * G * BS * 4;
+        const int step = unit * ATT_WARPS;
+        b += step;
+        pk += step * (BS * (D / 2));
+        s += step * (BS * NG * 2);
+        z += step * (BS * NG * 2);
+        sc += step * (G * BS * 4);
     }
 };
 
@@ -762,7 +765,11 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b_begin = split * blocks_per_split;
     const int b_end = split < ns ? min((int)nact, b_begin + blocks_per_split) : b_begin;      // CTAs x >= ns: dense recompute only
-    const int my_first = b_begin + 2 * warp;     // this warp's blocks: pairs my_first + 16 * it
+    // A warp takes pairs of blocks (fewer and wider copies, half the loop overhead), single blocks where a split has so
+    // few that pairs would leave warps idle (1000 tokens fp32: 47.3 -> 43.8 us a step; a line at 64 blocks measured the
+    // same).
+    const int unit = blocks_per_split <= ATT_WARPS ? 1 : 2, stride = unit * ATT_WARPS;
+    const int my_first = b_begin + unit * warp;     // this warp's units: my_first + stride * it
     char *ring = dsm, *wring = ring + warp * ATT_STAGES * LY::STAGE;
     char *qfrag = dsm + LY::RING_BYTES;
     float *wtile = reinterpret_cast<float *>(dsm + LY::RING_BYTES + LY::QFRAG + warp * LY::WTILE);
@@ -770,7 +777,7 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
 
     // start the pipeline before anything else
     AttIssuer<G, T2> issuer;
-    issuer.init(c, ws.token_scores, (int)nq, kv, sub, my_first, b_end, lane);
+    issuer.init(c, ws.token_scores, (int)nq, kv, sub, my_first, b_end, unit, lane);
 #pragma unroll
     for (int s = 0; s < ATT_STAGES - 1; ++s) issuer.issue(wring + s * LY::STAGE, lane);
 
@@ -829,7 +836,7 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
 
     // Softmax reference: the largest Phase-1 block maximum over the warp's blocks.  Weight scale F: the largest value
     // norm nu bounds a group's range by 2 nu, its INT4 scale by 2 nu / 15.
-    const int n_my = my_first < b_end ? (b_end - my_first + 2 * ATT_WARPS - 1) / (2 * ATT_WARPS) : 0;     // pairs
+    const int n_my = my_first < b_end ? (b_end - my_first + stride - 1) / stride : 0;     // units
     const bool have_mb = ws.m_b != nullptr, have4 = c.values_int4_packed != nullptr;
     const long mb_ld = ws.shard_chunk > 0 ? ws.shard_chunk : ws.ld;   // a rank's own rows of the exchange buffer
     float m_init = -INFINITY, F = 32768.0f;
@@ -837,7 +844,7 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
         float mx[HG], nu = 0.0f;
 #pragma unroll
         for (int g = 0; g < HG; ++g) mx[g] = -INFINITY;
-        for (int b = my_first + (lane >> 1) * (2 * ATT_WARPS) + (lane & 1); b < b_end && b < (int)nq; b += 32 * ATT_WARPS) {
+        for (int b = my_first + (lane / unit) * stride + lane % unit; b < b_end && b < (int)nq; b += 32 * ATT_WARPS) {
             if (have_mb) {
 #pragma unroll
                 for (int g = 0; g < HG; ++g) mx[g] = fmaxf(mx[g], ws.m_b[(long)(head0 + g) * mb_ld + b]);
@@ -852,8 +859,8 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
         float bound = warp_max(nu) * 0.135f;       // 2 / 15 with room for the rounding of values and scales to fp16
         if (have4 && !c.values_norm_max) {         // caches without norms: the scales themselves
             float s = 0.0f;
-            for (int i0 = 0; i0 < 2 * n_my; ++i0) {
-                const long b = my_first + (i0 >> 1) * (2 * ATT_WARPS) + (i0 & 1);
+            for (int i0 = 0; i0 < unit * n_my; ++i0) {
+                const long b = my_first + (i0 / unit) * stride + i0 % unit;
                 if (b >= b_end || b >= nq) break;
                 const __half2 *row = reinterpret_cast<const __half2 *>(c.values_int4_scales + ((long)kv * c.cap_tokens + b * BS) * NG);
                 for (int i = lane; i < BS * NG / 2; i += 32) { const float2 v = __half22float2(row[i]); s = fmaxf(s, fmaxf(fabsf(v.x), fabsf(v.y))); }
@@ -884,14 +891,14 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
         skip = __ballot_sync(FULL, f != 0);
     }
 
-    // Lane j keeps the key / value promotion bits of the warp's pair (it0 + j), one bit per head; they are re-read every
-    // 32 pairs.
-    unsigned my_masks = 0;   // km | vm << 8 of the pair's first block, the same << 16 of its second
+    // Lane j keeps the key / value promotion bits of the warp's unit (it0 + j), one bit per head; they are re-read every
+    // 32 units.
+    unsigned my_masks = 0;   // km | vm << 8 of the unit's first block, the same << 16 of its second
     const auto load_masks = [&](int it0) {
         my_masks = 0;
 #pragma unroll 1
-        for (int i = 0; i < 2; ++i) {
-            const int b = my_first + (it0 + lane) * (2 * ATT_WARPS) + i;
+        for (int i = 0; i < unit; ++i) {
+            const int b = my_first + (it0 + lane) * stride + i;
             unsigned km = 0, vm = 0;
             if (b < b_end) {
 #pragma unroll
@@ -906,13 +913,13 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
         }
     };
     load_masks(0);
-    // Tier-2 rows that will be needed are requested into L2 two pairs ahead (device memory only).
+    // Tier-2 rows that will be needed are requested into L2 two units ahead (device memory only).
     const auto prefetch = [&](int it) {
         const unsigned mk = __shfl_sync(FULL, my_masks, it & 31);
         if (mk == 0) return;
-        const long b = my_first + it * (2 * ATT_WARPS);
+        const long b = my_first + it * stride;
 #pragma unroll 1
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < unit; ++i) {
             const unsigned m = (mk >> (16 * i)) & 0xFFFFu;
             if ((m & 0xFFu) && !c.key_slots) prefetch_rows<T2>(t2_key_block<T2>(c, kv, b + i), lane);
             if ((m >> 8) && !c.value_slots) prefetch_rows<T2>(t2_value_block<T2>(c, kv, b + i), lane);
@@ -923,7 +930,7 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
 #pragma unroll 1
     for (int it = 0; it < n_my; ++it) {
         const unsigned pair_masks = __shfl_sync(FULL, my_masks, it & 31);
-        const int b0 = my_first + it * (2 * ATT_WARPS);
+        const int b0 = my_first + it * stride;
         char *st = wring + (it % ATT_STAGES) * LY::STAGE;
         const unsigned st_addr = wring_addr + (it % ATT_STAGES) * LY::STAGE;
         att_wait<ATT_STAGES - 2>();
@@ -931,7 +938,7 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
         issuer.issue(wring + ((it + ATT_STAGES - 1) % ATT_STAGES) * LY::STAGE, lane);
         if (((it + 2) & 31) > 1 && it + 2 < n_my) prefetch(it + 2);      // within the 32 pairs whose masks are at hand
 #pragma unroll 1
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < unit; ++i) {
             const int b = b0 + i;
             if (b >= b_end) break;
             const unsigned km = (pair_masks >> (16 * i)) & 0xFFu, vm = (pair_masks >> (16 * i + 8)) & 0xFFu;
