@@ -50,7 +50,7 @@ int attend_launch(const cqa_cache *c, const cqa_workspace *ws, const void *q, in
 
 int dense_launch(const cqa_cache *c, const cqa_workspace *ws, const void *q, int q_dtype, long num_tokens, float q_scale,
                  cudaStream_t st);
-int score_blocks_batched_launch(const cqa_batch_item *items_dev, int n_items, int kv_heads, int gqa_group, long max_nq,
+int score_blocks_batched_launch(const cqa_batch_item *items, const cqa_batch_item *items_dev, int n_items, int kv_heads, int gqa_group, long max_nq,
                                 int q_dtype, float q_scale, int do_append, cudaStream_t st);
 int selcert_batched_launch(const cqa_batch_item *items_dev, int n_items, int n_heads, long max_nq, const cqa_knobs *kn,
                            int q_dtype, int do_append, cudaStream_t st);
@@ -422,7 +422,7 @@ extern "C" int cqa_layer_step_batched(const cqa_batch_item *items, int n_items, 
                         "copy of the batch records");
     }
     if (rc) return rc;
-    rc = score_blocks_batched_launch(dev, n_items, c0.kv_heads, c0.gqa_group, max_nq, dtype, knobs->q_scale, do_append, st);
+    rc = score_blocks_batched_launch(items, dev, n_items, c0.kv_heads, c0.gqa_group, max_nq, dtype, knobs->q_scale, do_append, st);
     if (rc) return rc;
     rc = selcert_batched_launch(dev, n_items, c0.kv_heads * c0.gqa_group, max_nq, knobs, dtype, do_append, st);
     if (rc) return rc;
@@ -438,7 +438,8 @@ extern "C" int cqa_suggest_splits(int kv_heads, int gqa_group, int64_t nact, int
     }
     const int sms = sm_count();
     // Phase 2: two resident CTAs per SM, at least 8 blocks (one per warp) per split.
-    long target = ((long)sms * CQA_ATT_MIN_CTAS) / kv_heads;
+    const long rows = (long)kv_heads * (gqa_group == 8 ? 2 : 1);     // a CTA works on at most four heads
+    long target = ((long)sms * CQA_ATT_MIN_CTAS) / rows;
     if (target < 1) target = 1;
     long by_work = (nact + 7) / 8;
     long ns = target < by_work ? target : by_work;

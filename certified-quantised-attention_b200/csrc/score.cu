@@ -226,15 +226,14 @@ __global__ void __launch_bounds__(SCORE_WARPS * 32, 2) score_blocks_kernel(cqa_c
 // its blocks over all of grid.x.
 template <int G>
 __global__ void __launch_bounds__(SCORE_WARPS * 32, 2) score_blocks_batched_kernel(const cqa_batch_item *items, int q_dtype,
-                                                                                  float q_scale, int do_append)
+                                                                                  float q_scale, int do_append, int bpc)
 {
     grid_dependency_wait();      // the append kernel may be what writes the records
     const cqa_batch_item &it = *stage_batch_item(items + blockIdx.z);
     const long nq = (it.pos + do_append) / BS;
-    long bpc = (nq + gridDim.x - 1) / gridDim.x;
-    if (bpc < 2) bpc = 2;
+    if ((long)blockIdx.x * bpc >= nq) return;
     ScorePush none = {};
-    score_blocks_body<G>(it.cache, it.q, q_dtype, nq, q_scale, it.ws.m_b, it.ws.s_b, it.ws.ld, it.ws.token_scores, (int)bpc,
+    score_blocks_body<G>(it.cache, it.q, q_dtype, nq, q_scale, it.ws.m_b, it.ws.s_b, it.ws.ld, it.ws.token_scores, bpc,
                          it.ws.any_flags, 5 + it.cache.kv_heads * G, none);
 }
 
@@ -290,27 +289,34 @@ static int score_launch_g(const cqa_cache *c, const void *q, int q_dtype, long n
                       "score_blocks_kernel");
 }
 
-// Phase 1 of a batch: `max_nq` = most quantised blocks of any sequence.
-int score_blocks_batched_launch(const cqa_batch_item *items_dev, int n_items, int kv_heads, int gqa_group, long max_nq,
-                                int q_dtype, float q_scale, int do_append, cudaStream_t st)
+// Phase 1 of a batch; the sequences are split into runs of one length.
+int score_blocks_batched_launch(const cqa_batch_item *items, const cqa_batch_item *items_dev, int n_items, int kv_heads,
+                                int gqa_group, long max_nq, int q_dtype, float q_scale, int do_append, cudaStream_t st)
 {
-    // CTAs per (sequence, KV head): the count that minimises (waves of 2 CTAs per SM) x (blocks per CTA + a fixed
-    // start-up cost of about 16 blocks).  One CTA too many per head spills the grid into a second, nearly empty wave
-    // (5 instead of 4 CTAs per head cost 9 % of a 128K batch of 8); with many waves the granularity of a
-    // one-sequence launch is the best choice again.  The split does not change any result: blocks are independent.
-    const long slots = (long)sm_count() * 2, heads = (long)kv_heads * n_items;
+    // Blocks per CTA: the length that minimises the estimated end of the launch, with a fixed start-up cost of about 16
+    // blocks per CTA: one wave ends with its longest CTA, several (ragged lengths fill the SMs as they come free) with
+    // their total work and half of the longest.  The split does not change any result: blocks are independent.
+    const long slots = (long)sm_count() * 2;
     long p_max = (slots + kv_heads - 1) / kv_heads;          // what a launch for one sequence uses
     const long by_work = (max_nq + 15) / 16;                  // at least 16 blocks per CTA
     if (p_max > by_work) p_max = by_work;
     if (p_max < 1) p_max = 1;
-    long gx = 1;
+    long bpc = max_nq;
     double best = 0.0;
     for (long p = 1; p <= p_max; ++p) {
-        const long waves = (heads * p + slots - 1) / slots;
-        const double cost = (double)waves * ((double)((max_nq + p - 1) / p) + 16.0);
-        if (p == 1 || cost < best) { best = cost; gx = p; }
+        const long len = (max_nq + p - 1) / p;
+        double ctas = 0.0, work = 0.0;
+        for (int i = 0; i < n_items; ++i) {
+            const long nq = (items[i].pos + do_append) / BS, runs = (nq + len - 1) / len;
+            ctas += (double)runs * kv_heads;
+            work += ((double)nq + 16.0 * runs) * kv_heads;
+        }
+        const double longest = (double)len + 16.0;
+        const double cost = ctas <= slots ? longest : work / slots + 0.5 * longest;
+        if (p == 1 || cost < best) { best = cost; bpc = len; }
     }
-    dim3 grid((unsigned)gx, (unsigned)kv_heads, (unsigned)n_items);
+    if (bpc < 2) bpc = 2;
+    dim3 grid((unsigned)((max_nq + bpc - 1) / bpc), (unsigned)kv_heads, (unsigned)n_items);
 #define CQA_SCORE_BATCH_CASE(GG)                                                                                       \
     case GG: {                                                                                                         \
         constexpr int SMEM = SCORE_SMEM + GG * D * 4 + SCORE_WARPS * 2 * 8;                                            \
@@ -319,7 +325,7 @@ int score_blocks_batched_launch(const cqa_batch_item *items_dev, int n_items, in
                                   "cudaFuncSetAttribute(score_blocks_batched_kernel)");                                \
         if (rc) return rc;                                                                                             \
         return check_cuda(launch_chained(score_blocks_batched_kernel<GG>, grid, dim3(SCORE_WARPS * 32), SMEM, st, true, \
-                                         items_dev, q_dtype, q_scale, do_append), "score_blocks_batched_kernel");      \
+                                         items_dev, q_dtype, q_scale, do_append, (int)bpc), "score_blocks_batched_kernel");      \
     }
     switch (gqa_group) {
         CQA_SCORE_BATCH_CASE(1)
