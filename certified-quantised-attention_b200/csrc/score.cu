@@ -70,6 +70,62 @@ __device__ __forceinline__ float chain8_f2(const float2 (&a)[4], const float2 (&
     return __fadd_rn(p.x, p.y);
 }
 
+// cexp (common.cuh) of two values <= 0, bit for bit: the same operations on packed operands, with the nearest integer
+// from the 2^23 trick (exact for |t| < 2^22; the product is scalar because a packed product and a packed add behind it
+// are merged into one rounding) and its bits as the exponent.
+__device__ __forceinline__ float2 cexp2_nonpositive(float2 x)
+{
+    const float2 lo = make_float2(fmaxf(x.x, -104.0f), fmaxf(x.y, -104.0f));
+    const float2 magic = make_float2(12582912.0f, 12582912.0f), nmagic = make_float2(-12582912.0f, -12582912.0f);
+    const float2 m = __fadd2_rn(make_float2(__fmul_rn(lo.x, 1.44269504088896341f), __fmul_rn(lo.y, 1.44269504088896341f)), magic);
+    const float2 n = __fadd2_rn(m, nmagic);
+    float2 r = __ffma2_rn(n, make_float2(-0.693145751953125f, -0.693145751953125f), lo);
+    r = __ffma2_rn(n, make_float2(-1.42860682030941723212e-6f, -1.42860682030941723212e-6f), r);
+    float2 p = make_float2(1.9875691500e-4f, 1.9875691500e-4f);
+    p = __ffma2_rn(p, r, make_float2(1.3981999507e-3f, 1.3981999507e-3f));
+    p = __ffma2_rn(p, r, make_float2(8.3334519073e-3f, 8.3334519073e-3f));
+    p = __ffma2_rn(p, r, make_float2(4.1665795894e-2f, 4.1665795894e-2f));
+    p = __ffma2_rn(p, r, make_float2(1.6666665459e-1f, 1.6666665459e-1f));
+    p = __ffma2_rn(p, r, make_float2(5.0000001201e-1f, 5.0000001201e-1f));
+    p = __ffma2_rn(p, make_float2(__fmul_rn(r.x, r.x), __fmul_rn(r.y, r.y)), r);
+    p = __fadd2_rn(p, make_float2(1.0f, 1.0f));
+    // 2^n in two factors below 2^-126 (the second is one otherwise)
+    const auto scale = [](float v, float bits, float x0) {
+        int ni = __float_as_int(bits);
+        asm("" : "+r"(ni));      // without this the shift below was dropped for the first of the pair (nvcc 12.9)
+        ni -= 0x4B400000;
+        const bool low = ni < -126;
+        v = __fmul_rn(v, __int_as_float(((low ? ni + 64 : ni) + 127) << 23));
+        v = low ? __fmul_rn(v, 5.42101086242752217e-20f) : v;
+        return x0 > -104.0f ? v : 0.0f;
+    };
+    return make_float2(scale(p.x, m.x, x.x), scale(p.y, m.y, x.y));
+}
+
+// Sum (or maximum) over the 16 lanes of a half warp of GH values per lane at once, with the strides 8, 4, 2, 1 of hw_sum:
+// a lane keeps the values with the bits of its number, so lane L ends with value L / (16 / GH) (the lanes of one value
+// agree bit for bit: every addition has the same two operands as the all-reduce, in either order).
+template <int GH, bool MAX>
+__device__ __forceinline__ float half_warp_reduce(float (&v)[GH], int L)
+{
+    const auto op = [](float a, float b) { return MAX ? fmaxf(a, b) : __fadd_rn(a, b); };
+    int stride = 8;
+#pragma unroll
+    for (int w = GH / 2; w >= 1; w >>= 1) {
+        const bool up = (L & stride) != 0;
+#pragma unroll
+        for (int i = 0; i < w; ++i) v[i] = op(up ? v[i + w] : v[i], __shfl_xor_sync(FULL, up ? v[i] : v[i + w], stride));
+        stride >>= 1;
+    }
+    float r = v[0];
+#pragma unroll
+    for (int o = 8 / GH; o >= 1; o >>= 1) r = op(r, __shfl_xor_sync(FULL, r, o));
+    return r;
+}
+// Value i of half_warp_reduce in every lane of the half warp.
+template <int GH>
+__device__ __forceinline__ float half_warp_get(float r, int i, int lane) { return __shfl_sync(FULL, r, (lane & 16) + i * (16 / GH)); }
+
 template <int G>
 __device__ __forceinline__ void score_blocks_body(const cqa_cache &c, const void *q, int q_dtype, long nq, float q_scale,
                                                   float *m_b, float *s_b, long ld, float *tok, int blocks_per_cta,
@@ -119,7 +175,7 @@ __device__ __forceinline__ void score_blocks_body(const cqa_cache &c, const void
         const char *kb = sbase + half * BLOCK_BYTES;
         const float *sc = reinterpret_cast<const float *>(sbase + ST_SCALES) + half * D;
         const float *zp = reinterpret_cast<const float *>(sbase + ST_ZEROS) + half * D;
-#pragma unroll
+#pragma unroll 1
         for (int pass = 0; pass < G / GH; ++pass) {
             float2 qs[GH][4];
             float zq[GH];
@@ -133,9 +189,15 @@ __device__ __forceinline__ void score_blocks_body(const cqa_cache &c, const void
                     load8<float>(s_q + (pass * GH + g) * D + 8 * L, qv);
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
-                        qs[g][i] = make_float2(__fmul_rn(qv[2 * i], sg[2 * i]), __fmul_rn(qv[2 * i + 1], sg[2 * i + 1]));
-                    zq[g] = hw_sum(chain8(qv, zz));
+                        qs[g][i] = __fmul2_rn(make_float2(qv[2 * i], qv[2 * i + 1]), make_float2(sg[2 * i], sg[2 * i + 1]));
+                    float2 q2[4], z2[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { q2[i] = make_float2(qv[2 * i], qv[2 * i + 1]); z2[i] = make_float2(zz[2 * i], zz[2 * i + 1]); }
+                    zq[g] = chain8_f2(q2, z2);
                 }
+                const float zr = half_warp_reduce<GH, false>(zq, L);
+#pragma unroll
+                for (int g = 0; g < GH; ++g) zq[g] = half_warp_get<GH>(zr, g, lane);
             }
             // Tokens are visited in pairs (j^L, (j+8)^L): the first step of the 16-lane reduce-scatter
             // (stride 8) is applied at once, so only 8 partial sums per head stay live.
@@ -154,6 +216,7 @@ __device__ __forceinline__ void score_blocks_body(const cqa_cache &c, const void
                     acc[g][j] = __fadd_rn(lo, __shfl_xor_sync(FULL, hi, 8));
                 }
             }
+            float score[GH];
 #pragma unroll
             for (int g = 0; g < GH; ++g) {
 #pragma unroll
@@ -161,18 +224,34 @@ __device__ __forceinline__ void score_blocks_body(const cqa_cache &c, const void
 #pragma unroll
                 for (int j = 0; j < 2; ++j) acc[g][j] = __fadd_rn(acc[g][j], __shfl_xor_sync(FULL, acc[g][j + 2], 2));
                 acc[g][0] = __fadd_rn(acc[g][0], __shfl_xor_sync(FULL, acc[g][1], 1));
-                const float score = __fmul_rn(__fadd_rn(acc[g][0], zq[g]), q_scale);
-                const float mx = hw_max(score);
-                const float e = cexp(__fsub_rn(score, mx));
-                const float ssum = hw_sum(e);
-                if (live) {
-                    const int gg = pass * GH + g;
-                    if (tok) tok[(((long)kv * nq + b) * G + gg) * BS + L] = score;
-                    if (L == 0) {
-                        const long o = (long)(kv * G + gg) * ld + b;
-                        m_b[o] = mx;
-                        s_b[o] = ssum;
-                    }
+                score[g] = __fmul_rn(__fadd_rn(acc[g][0], zq[g]), q_scale);
+                zq[g] = score[g];
+            }
+            const float mr = half_warp_reduce<GH, true>(zq, L);
+            float e[GH];
+            if constexpr (GH >= 2) {
+#pragma unroll
+                for (int g = 0; g < GH; g += 2) {
+                    const float2 x = cexp2_nonpositive(make_float2(__fsub_rn(score[g], half_warp_get<GH>(mr, g, lane)),
+                                                                   __fsub_rn(score[g + 1], half_warp_get<GH>(mr, g + 1, lane))));
+                    e[g] = x.x;
+                    e[g + 1] = x.y;
+                }
+            } else {
+                e[0] = cexp(__fsub_rn(score[0], mr));
+            }
+            const float sr = half_warp_reduce<GH, false>(e, L);
+            if (live) {
+                if (tok) {
+                    float *t = tok + (((long)kv * nq + b) * G + pass * GH) * BS + L;
+#pragma unroll
+                    for (int g = 0; g < GH; ++g) t[g * BS] = score[g];
+                }
+                // the lanes of a head hold its maximum and sum; one of them stores each
+                if (L % (16 / GH) == 0) {
+                    const long o = (long)(kv * G + pass * GH + L / (16 / GH)) * ld + b;
+                    m_b[o] = mr;
+                    s_b[o] = sr;
                 }
             }
         }
