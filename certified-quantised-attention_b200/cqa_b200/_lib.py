@@ -29,7 +29,7 @@ SYMBOLS = [
     "cqa_step_stats",
 ]
 PARTIAL_STRIDE = 130
-STATS_PARTS = 16
+SUMMARY_ITEMS = 32
 
 vp = C.c_void_p
 
@@ -206,7 +206,7 @@ def lib() -> C.CDLL:
     L.cqa_peer_buffer_bytes.restype = C.c_int64
     L.cqa_prefill_encode.argtypes = [C.POINTER(CqaPrefillItem), i32, i32, vp]
     L.cqa_layer_step_batched.argtypes = [C.POINTER(CqaBatchItem), i32, vp, pk, i32, i32, vp]
-    L.cqa_step_stats.argtypes = [pc, pw, i64, i64, vp, vp]
+    L.cqa_step_stats.argtypes = [pc, pw, i64, i64, vp, vp, vp]
     L.cqa_wait_timeouts.argtypes = [C.POINTER(C.c_int), i32]
     L.cqa_launch_count.argtypes = [i32]
     L.cqa_launch_count.restype = C.c_int64

@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from cqa_b200 import _lib
-from dotcache.kernels.tiered_kv_cache import TieredKeyCacheLayer
+from dotcache.kernels.tiered_kv_cache import TieredKeyCacheLayer, _get_device, _raw_stream
 
 DEFAULT_V_TOLERANCE = 0.5
 TOP_K_BLOCKS = 4
@@ -47,6 +47,7 @@ class _Workspace:
     """Device buffers for one layer's step, kept in cache._certified_workspace."""
 
     _serial = 0
+    _version = 0        # counts the replaced buffers
 
     def draw_seed(self) -> int:
         """Key of this workspace's Philox stream: torch.initial_seed() mixed (splitmix64) with the workspace's
@@ -85,14 +86,14 @@ class _Workspace:
         self.dense_m = torch.empty(H, self.dense_splits, **f32)
         self.dense_l = torch.empty(H, self.dense_splits, **f32)
         self.dense_acc = torch.empty(H, self.dense_splits, 128, **f32)
-        # certificate structs, the flag words (4 flags, dense-head count and list) and the telemetry words of
-        # cqa_step_stats: one D2H copy reads all three
+        # certificate structs followed by the flag words (4 flags, dense-head count and list):
+        # one D2H copy reads both; behind them the scratch words of cqa_step_stats
         self.cert_bytes = H * _lib.CERT_BYTES
         self.stats_off = self.cert_bytes + 4 * (5 + H)
-        self.cert_buf = torch.zeros(self.stats_off + 4 * (2 * H + 2 * cache.kv_heads + _lib.STATS_PARTS), **u8)
+        self.cert_buf = torch.zeros(self.stats_off + 4 * (2 * H + 2 * cache.kv_heads + 17), **u8)
+        self.summary = None
         self.out = torch.empty(H, 128, **f32)
         self.tickets = torch.zeros(cache.kv_heads + H, dtype=torch.int32, device=device)
-        self.cert_host = None
         self._u_flat = None
         self._step_in = None
         # In-kernel exploration draw: torch's seed mixed with a per-workspace serial number, so that the layers of
@@ -159,23 +160,14 @@ class _Workspace:
                     "sorted_idx", "sorted_cumsum", "part_m", "part_l", "part_acc", "dense_m", "dense_l", "dense_acc",
                     "cert_buf", "out", "tickets", "sel_width"):
             object.__setattr__(self, "_struct_stale", True)
+            object.__setattr__(self, "_version", self._version + 1)
         object.__setattr__(self, name, value)
-
-    def _read_back(self) -> np.ndarray:
-        """The certificate buffer on the host (synchronises), through a pinned buffer that is kept."""
-        buf = self.cert_buf
-        host = self.cert_host
-        if host is None or host.numel() != buf.numel():
-            host = self.cert_host = torch.empty(buf.numel(), dtype=torch.uint8, pin_memory=True)
-        host.copy_(buf, non_blocking=True)
-        torch.cuda.current_stream(buf.device).synchronize()
-        return host.numpy()
 
     def read_cert(self) -> tuple[dict, list]:
         """Copy the certificate structs and flags to the host (synchronises)."""
-        host = self._read_back()
+        host = self.cert_buf[: self.stats_off].cpu().numpy()
         arr = np.frombuffer(host[: self.cert_bytes].tobytes(), dtype=_CERT_DTYPE)
-        flags = np.frombuffer(host[self.cert_bytes: self.stats_off].tobytes(), dtype=np.int32).tolist()
+        flags = np.frombuffer(host[self.cert_bytes:].tobytes(), dtype=np.int32).tolist()
         cols: dict[str, Any] = {f: arr[f].astype(np.int64) for f in _CERT_INT_FIELDS}
         for f in _CERT_F32_FIELDS:
             cols[f] = arr[f].astype(np.float64)
@@ -718,6 +710,14 @@ def certified_attention_layer(
     `torch.initial_seed()`, a per-workspace serial number and a per-cache call
     counter, so different layers draw different sets).
     """
+    key = (gqa_group, q_scale, v_tolerance, top_k_fp16_keys, ranking_fallback, ranking_r, ranking_fallback_mode, tau_cov, k_min,
+           k_max, rung1_threshold, rung1_multiplier, score_consistency_check, eps_guard, exploration_rate, value_error_mode,
+           per_kv_group_topk)
+    plan = cache._layer_plan
+    if plan is not None and plan.key == key and phase_timings is None and exploration_uniforms is None:
+        stream = plan.ready(cache, q_all)
+        if stream is not None:
+            return plan.step(cache, q_all, stream, exploration_generator, collect_stats)
     if not q_all.is_cuda:
         raise RuntimeError("certified_attention_layer needs CUDA tensors; there is no CPU fallback")
     if value_error_mode not in ("loose", "tight"):
@@ -798,6 +798,9 @@ def certified_attention_layer(
     ws.ensure_sel_width(_selection_width(k_max, rung1_threshold, rung1_multiplier, nq), device)
     wstruct = ws.fill_struct(nact)
 
+    if phase_timings is None and exploration_uniforms is None:
+        cache._layer_plan = _LayerPlan(key, cache, ws, q, knobs, float(exploration_rate), (k_max, rung1_threshold, rung1_multiplier))
+
     u_ptr, u_ld = None, 0
     u_keep = None
     if exploration_rate > 0.0:
@@ -843,7 +846,7 @@ def certified_attention_layer(
     output = ws.out
     if not collect_stats:
         return output, {}
-    stats = _assemble_stats(
+    return output, _assemble_stats(
         cache, ws, H, G, nq, nact, has_int4=has_int4, force_trailing=force_trailing_value_fp16,
         tau_cov=tau_cov, rung1_threshold=rung1_threshold, rung1_multiplier=rung1_multiplier,
         exploration_rate=exploration_rate, score_consistency_check=score_consistency_check,
@@ -851,7 +854,84 @@ def certified_attention_layer(
         ranking_fallback_mode=ranking_fallback_mode, top_k_fp16_keys=top_k_fp16_keys,
         value_error_mode=value_error_mode,
     )
-    return output, stats
+
+
+class _LayerPlan:
+    """What `certified_attention_layer` works out anew for a cache only when its arguments, buffers or block count
+    change: the structs of the library call, with a private workspace struct.  A decode loop calls it with the same
+    settings every step, and the 16 us the interpreter took for them were half of a short context's step."""
+
+    __slots__ = ("key", "ws", "version", "splits", "desc", "w", "refs", "knobs", "qd", "dtype", "shape", "dev", "rate", "width_args",
+                 "nq", "trailing", "can_force", "u", "out", "fn")
+
+    def __init__(self, key, cache, ws, q, knobs, rate, width_args):
+        self.key, self.ws, self.version = key, ws, ws._version
+        self.splits = (ws.num_splits, ws.dense_splits)
+        self.desc = cache._desc(int(key[0]))
+        self.w = _lib.CqaWorkspace.from_buffer_copy(bytes(ws.struct))
+        self.qd, self.dtype, self.shape, self.dev = _lib.dtype_code(q.dtype), q.dtype, q.shape, q.get_device()
+        self.rate, self.width_args = rate, width_args
+        if rate > 0.0:
+            self.w.rng_seed = ws.draw_seed()
+        self.can_force = bool(
+            cache.values_int4_packed is not None and cache.values_fp16_gpu is not None
+            and (cache.values_fp16_cpu is not None or cache.fp16_value_cache_capacity is None or cache.static_resident_value_cache))
+        flip = _lib.CqaKnobs.from_buffer_copy(bytes(knobs))
+        flip.force_trailing_value_fp16 = 1 - knobs.force_trailing_value_fp16
+        pair = (knobs, flip) if not knobs.force_trailing_value_fp16 else (flip, knobs)
+        self.knobs = (pair, C.byref(pair[0]), C.byref(pair[1]))
+        self.refs = (C.byref(self.desc), C.byref(self.w))
+        self.nq, self.trailing, self.u, self.out = -1, None, None, ws.out
+        self.fn = _lib.lib().cqa_layer_step
+
+    def ready(self, cache, q):
+        """The stream to run on, or None when the plan does not describe this call."""
+        ws = self.ws
+        if (cache._certified_workspace.get("cqa_ws") is not ws or ws._version != self.version
+                or (ws.num_splits, ws.dense_splits) != self.splits or cache._desc_cache.get(self.desc.gqa_group) is not self.desc
+                or q.dtype is not self.dtype or q.shape != self.shape or not q.is_cuda or q.get_device() != self.dev
+                or not q.is_contiguous() or _get_device() != self.dev):
+            return None
+        nq = cache.num_quantized_blocks
+        trailing = cache.num_tokens % cache.block_size != 0
+        if nq != self.nq or trailing is not self.trailing:
+            if nq <= 0 or _selection_width(*self.width_args, nq) > ws.sel_width:
+                return None
+            nact = nq + (1 if trailing else 0)
+            # as in fill_struct: never more splits than eight-block groups of work
+            self.w.num_splits = max(1, min(self.splits[0], (nact + 7) // 8))
+            self.w.dense_splits = max(1, min(self.splits[1], (nact + 7) // 8))
+            self.nq, self.trailing, self.u = nq, trailing, None
+        return _raw_stream(self.dev)
+
+    def step(self, cache, q, stream, generator, collect_stats):
+        ws, nq = self.ws, self.nq
+        u_ptr, u_ld = None, 0
+        if self.rate > 0.0:
+            if generator is not None:
+                if self.u is None:
+                    view = ws.uniform_buffer(nq, q.device)
+                    self.u = (view, view.data_ptr(), view.shape)
+                torch.rand(self.u[2], generator=generator, out=self.u[0])
+                u_ptr, u_ld = self.u[1], nq
+            else:
+                self.w.rng_offset = ws.rng_calls
+                ws.rng_calls += 1
+        rc = self.fn(self.refs[0], self.knobs[2 if self.trailing and self.can_force else 1], self.refs[1], q.data_ptr(), self.qd,
+                     cache.num_tokens, nq, u_ptr, u_ld, stream)
+        if rc:
+            _lib.check(rc, "cqa_layer_step")
+        nact = nq + (1 if self.trailing else 0)
+        if cache._hot is not None:
+            cache._hot_tier_update(self.desc, self.w, nact, stream)
+        if not collect_stats:
+            return self.out, {}
+        (G, _q, _v, top_k, fallback, r, mode, tau, _k1, _k2, thr, mult, check, eps, rate, value_mode, _g) = self.key
+        return self.out, _assemble_stats(
+            cache, ws, self.shape[0], int(G), nq, nact, has_int4=cache.values_int4_packed is not None,
+            force_trailing=self.trailing and self.can_force, tau_cov=tau, rung1_threshold=thr, rung1_multiplier=mult,
+            exploration_rate=rate, score_consistency_check=check, eps_guard=eps, ranking_fallback=fallback, ranking_r=r,
+            ranking_fallback_mode=mode, top_k_fp16_keys=top_k, value_error_mode=value_mode)
 
 
 def _flush_timers(timings, pending):
@@ -879,35 +959,28 @@ def _assemble_stats(cache, ws: _Workspace, H, G, nq, nact, *, has_int4, force_tr
                     rung1_threshold, rung1_multiplier, exploration_rate, score_consistency_check, eps_guard,
                     ranking_fallback, ranking_r, ranking_fallback_mode, top_k_fp16_keys,
                     value_error_mode) -> dict[str, Any]:
-    """The reference's per-layer stats dict (certified_attention.py:2608-2788).  One telemetry kernel behind the step
-    and one copy of the certificate buffer; everything after that is host arithmetic on short lists."""
-    KV = cache.kv_heads
+    """The reference's per-layer stats dict (certified_attention.py:2608-2788), from the summary that one launch behind
+    the step writes into pinned memory (cqa_step_stats)."""
     dev = ws.cert_buf.device
+    if ws.summary is None:
+        buf = torch.empty(_lib.SUMMARY_ITEMS, dtype=torch.float64, pin_memory=True)
+        ws.summary = (buf, buf.numpy())
     with _lib.on_device(dev):
         _lib.check(_lib.lib().cqa_step_stats(C.byref(cache._desc(G)), C.byref(ws.struct), nq, nact,
-                                             ws.cert_buf.data_ptr() + ws.stats_off, _lib.current_stream(dev)),
-                   "cqa_step_stats")
-    host = ws._read_back()
-    arr = np.frombuffer(host, dtype=_CERT_DTYPE, count=H)
-    flag2 = int(host[ws.cert_bytes + 8: ws.cert_bytes + 12].view(np.int32)[0])
-    tele_i = host[ws.stats_off:].view(np.int32)
-    tele_f = host[ws.stats_off:].view(np.float32)
-    col = lambda name: arr[name].tolist()  # noqa: E731
-    mean = lambda v: sum(v) / len(v)  # noqa: E731
-    rung4 = bool(score_consistency_check and flag2)
+                                             ws.cert_buf.data_ptr() + ws.stats_off, ws.summary[0].data_ptr(),
+                                             _lib.current_stream(dev)), "cqa_step_stats")
+    v = ws.summary[1].tolist()
+    (_, violation_heads, boundary_heads, rung1_heads, head_blocks, dense_heads, explored, disagree_r1, disagree_r3) = map(int, v[:9])
+    rung4 = bool(score_consistency_check and v[0])
     kb, vb = _vram_stats(cache)
     total_blocks = H * cache.num_blocks
-    delta = col("delta")
-    violation_heads = sum(col("consistency_violation"))
-    boundary_heads = sum(col("boundary_triggered"))
-    rung1_heads = sum(col("rung1_triggered"))
     if rung4:
         # every head was recomputed densely; same keys as the reference's early return (:1771-1796)
         return {
             "total_blocks": total_blocks, "skipped_blocks": 0, "skip_rate": 0.0,
             "attended_blocks": total_blocks, "v_format": "fp16",
             "score_consistency_violation_heads": violation_heads,
-            "delta_bound_mean": mean(delta), "eps_guard": float(eps_guard),
+            "delta_bound_mean": v[12] / H, "eps_guard": float(eps_guard),
             "h2d_key_bytes": 0, "h2d_key_blocks": 0, "h2d_value_bytes": 0, "h2d_value_blocks": 0,
             "h2d_total_bytes": 0, "vram_fp16_key_cache_bytes": kb, "vram_fp16_value_cache_bytes": vb,
             "rung1_fired": bool(rung1_heads > 0), "rung2_fired": False, "rung3_fired": False,
@@ -915,15 +988,15 @@ def _assemble_stats(cache, ws: _Workspace, H, G, nq, nact, *, has_int4, force_tr
             "boundary_check_triggered_heads": boundary_heads,
             "boundary_check_fired": bool(boundary_heads > 0),
         }
-    skipped = int(tele_i[:H].sum())
-    head_blocks = sum(col("value_promoted_blocks")) if has_int4 else 0
-    union_blocks = int(tele_i[2 * H + 2 * KV:].sum()) if (has_int4 and head_blocks) else 0
+    skipped = int(v[26])
+    if not has_int4:
+        head_blocks = 0
+    union_blocks = int(v[31]) if head_blocks else 0
     if has_int4:
         v_format = "mixed" if (head_blocks or force_trailing) else "int4"
     else:
         v_format = "fp16"
     rung2 = bool(has_int4 and v_format == "mixed")
-    dense_heads = sum(col("dense"))
     stats: dict[str, Any] = {
         "total_blocks": total_blocks, "skipped_blocks": skipped,
         "skip_rate": float(skipped) / float(total_blocks), "attended_blocks": total_blocks - skipped,
@@ -975,55 +1048,49 @@ def _assemble_stats(cache, ws: _Workspace, H, G, nq, nact, *, has_int4, force_tr
     stats["rung3_fired"] = bool(dense_heads > 0)
     stats["rung4_fired"] = False
     if has_int4:
-        rho = tele_f[H: 2 * H].tolist()
-        rho_max = max(rho)
-        eta_int4 = max(tele_f[2 * H: 2 * H + KV].tolist())
+        rho_max, eta_int4 = v[28], v[29]
         stats["rho_max"] = rho_max
-        stats["rho_mean"] = mean(rho)
+        stats["rho_mean"] = v[27] / H
         stats["eta_int4"] = eta_int4
         stats["int4_error_bound_loose"] = eta_int4 * rho_max
         stats["int4_error_bound"] = stats["int4_error_bound_loose"]
-        e_val, e_pre = col("e_val"), col("e_pre")
-        stats["e_val_max"] = max(e_val)
-        stats["e_val_mean"] = mean(e_val)
+        stats["e_val_max"] = v[14]
+        stats["e_val_mean"] = v[13] / H
         stats["value_error_mode"] = value_error_mode
-        stats["e_val_pre_rung2_max"] = max(e_pre)
-        stats["e_val_pre_rung2_mean"] = mean(e_pre)
+        stats["e_val_pre_rung2_max"] = v[16]
+        stats["e_val_pre_rung2_mean"] = v[15] / H
         if head_blocks:
             stats["value_fallback_blocks"] = union_blocks
             stats["value_fallback_head_blocks"] = head_blocks
-    ks, tail = col("k_star"), col("tail_mass")
-    stats["k_star_mean"] = mean(ks)
-    stats["k_star_min"] = min(ks)
-    stats["k_star_max"] = max(ks)
+    stats["k_star_mean"] = v[9] / H
+    stats["k_star_min"] = int(v[10])
+    stats["k_star_max"] = int(v[11])
     stats["tau_cov"] = float(tau_cov) if tau_cov is not None else 0.0
-    stats["tau_cov_actual_mean"] = mean(col("tau_actual"))
-    stats["tail_mass_int8_est_mean"] = mean(tail)
-    stats["tail_mass_int8_est_max"] = max(tail)
+    stats["tau_cov_actual_mean"] = v[17] / H
+    stats["tail_mass_int8_est_mean"] = v[18] / H
+    stats["tail_mass_int8_est_max"] = v[19]
     stats["rung1_triggered_heads"] = rung1_heads
     stats["rung1_threshold"] = float(rung1_threshold) if rung1_threshold is not None else -1.0
     stats["rung1_multiplier"] = float(rung1_multiplier)
     stats["exploration_rate"] = float(exploration_rate)
-    stats["exploration_blocks"] = sum(col("exploration_blocks"))
-    v_max_layer = max(tele_f[2 * H + KV: 2 * H + 2 * KV].tolist())
+    stats["exploration_blocks"] = explored
+    v_max_layer = v[30]
     stats["v_max_layer"] = v_max_layer
     have_delta = (ranking_fallback or score_consistency_check) and nq > 0
     if have_delta and v_max_layer > 0.0:
-        e2d = np.exp(2.0 * arr["delta"])
-        e_key = 2.0 * v_max_layer * e2d * arr["tail_mass"] * (e2d - 1.0)
-        stats["e_key_step_mean"] = float(e_key.mean())
-        stats["e_key_step_max"] = float(e_key.max())
+        stats["e_key_step_mean"] = v_max_layer * v[24] / H
+        stats["e_key_step_max"] = v_max_layer * v[25]
     if score_consistency_check:
         stats["score_consistency_violation_heads"] = violation_heads
-        stats["delta_bound_mean"] = mean(delta)
+        stats["delta_bound_mean"] = v[12] / H
         stats["eps_guard"] = float(eps_guard)
         stats["rung4_fired"] = False
         stats["rung4_violating_heads"] = 0
     if ranking_fallback:
         rk = min(max(int(ranking_r), int(top_k_fp16_keys or 0), 4), nq)
         stats["ranking_heads_total"] = H
-        stats["ranking_disagree_r1"] = sum(col("ranking_disagree_r1"))
-        stats["ranking_disagree_r3"] = sum(col("ranking_disagree_r3"))
+        stats["ranking_disagree_r1"] = disagree_r1
+        stats["ranking_disagree_r3"] = disagree_r3
         stats["ranking_fallback_triggered"] = dense_heads
         stats["ranking_r"] = int(ranking_r)
         stats["ranking_k"] = int(rk)
@@ -1031,11 +1098,10 @@ def _assemble_stats(cache, ws: _Workspace, H, G, nq, nact, *, has_int4, force_tr
         stats["boundary_check_triggered_heads"] = boundary_heads
         stats["boundary_check_fired"] = bool(boundary_heads > 0)
         if rk >= 2:
-            gap = (arr["fp16_top1"] - arr["fp16_top2"]).tolist()
-            stats["score_gap_top12_mean"] = mean(gap)
-            stats["score_gap_top12_min"] = min(gap)
-        stats["s_int8_top1_mean"] = mean(col("int8_top1"))
-        stats["s_fp16_top1_mean"] = mean(col("fp16_top1"))
+            stats["score_gap_top12_mean"] = v[22] / H
+            stats["score_gap_top12_min"] = v[23]
+        stats["s_int8_top1_mean"] = v[20] / H
+        stats["s_fp16_top1_mean"] = v[21] / H
     return stats
 
 

@@ -31,6 +31,10 @@ from cqa_b200 import _lib
 BLOCK = 16
 HEAD_DIM = 128
 
+# the current device and its current stream without torch's checks (a CUDA tensor at hand means CUDA is initialised)
+_get_device = getattr(torch._C, "_cuda_getDevice", None)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
 
 def _require_cuda(t: torch.Tensor, what: str) -> None:
     if not t.is_cuda:
@@ -110,6 +114,7 @@ class TieredKeyCacheLayer:
     _certified_workspace: dict = field(default_factory=dict, repr=False)
     _desc_cache: dict = field(default_factory=dict, repr=False)
     _hot: dict | None = field(default=None, repr=False)     # bounded hot tier: tables, counters, struct
+    _layer_plan: Any = field(default=None, repr=False)      # certified_attention_layer: what the last call worked out
 
     # ------------------------------------------------------------------ C ABI view
 
@@ -335,25 +340,34 @@ class TieredKeyCacheLayer:
         Reference: tiered_kv_cache.py:545-708 (append_token, _quantize_block,
         _quantize_value_block)."""
         pos = self.num_tokens
-        if pos >= self.keys_int8.shape[1]:
+        plan = self._desc_cache.get("append")
+        if plan is None:
+            plan = self._desc_cache["append"] = (C.byref(self._desc()), int(self.keys_int8.shape[1]), self.kv_heads * self.head_dim,
+                                                 _lib.lib().cqa_append_token)
+        desc, cap, numel, entry = plan
+        if pos >= cap:
             raise ValueError(
-                f"cache capacity {self.keys_int8.shape[1]} exhausted; build the cache with a larger max_new_tokens")
-        _require_cuda(key_fp16, "key")
-        k = key_fp16.reshape(self.kv_heads, self.head_dim)
-        v = value_fp16.reshape(self.kv_heads, self.d_v)
+                f"cache capacity {cap} exhausted; build the cache with a larger max_new_tokens")
+        k, v = key_fp16, value_fp16
+        if not k.is_cuda:
+            _require_cuda(k, "key")
+        if k.numel() != numel or v.numel() != numel:      # raises
+            k, v = k.reshape(self.kv_heads, self.head_dim), v.reshape(self.kv_heads, self.d_v)
         if v.dtype != k.dtype:
             v = v.to(k.dtype)
         if not k.is_contiguous():
             k = k.contiguous()
         if not v.is_contiguous():
             v = v.contiguous()
-        defer = self._defer_int4_flag()
-        dev = k.device
-        with _lib.on_device(dev):
-            rc = _lib.lib().cqa_append_token(
-                C.byref(self._desc()), k.data_ptr(), v.data_ptr(), _lib.dtype_code(k.dtype), pos,
-                1 if defer else 0, _lib.current_stream(dev))
-        _lib.check(rc, "cqa_append_token")
+        dev = k.get_device()
+        args = (desc, k.data_ptr(), v.data_ptr(), _lib.dtype_code(k.dtype), pos, 1 if self._defers_int4() else 0)
+        if _get_device() == dev:
+            rc = entry(*args, _raw_stream(dev))
+        else:
+            with _lib.on_device(k.device):
+                rc = entry(*args, _raw_stream(dev))
+        if rc:
+            _lib.check(rc, "cqa_append_token")
         self._advance_after_append(pos)
 
     # ------------------------------------------------------------------ bounded hot tier

@@ -264,12 +264,19 @@ typedef struct {
 } cqa_prefill_item;
 int cqa_prefill_encode(const cqa_prefill_item *items, int n_items, int src_dtype, void *stream);
 
-/* Telemetry of the step whose masks and mass fractions are in `ws`, for hosts that assemble statistics: `out` takes
- * 2 * H + 2 * KV + CQA_STATS_PARTS 4-byte words: [H] int32 blocks outside the FP16-key mask, [H] float32 sums of the
- * mass fractions, [KV] float32 largest eta_b, [KV] float32 largest nu_b of the active blocks, [CQA_STATS_PARTS] int32
- * counts (to be added up) of blocks that at least one head reads from the Tier-2 values. */
-#define CQA_STATS_PARTS 16
-int cqa_step_stats(const cqa_cache *c, const cqa_workspace *ws, int64_t nq, int64_t nact, void *out, void *stream);
+/* Telemetry of the step whose masks, mass fractions and certificate are in `ws`, for hosts that assemble statistics:
+ * one launch, then a wait for the stream.  `scratch`: 2 * (H + KV) + 17 words on the device, zeroed once.
+ * `summary_host` (pinned): CQA_SUMMARY_ITEMS doubles:
+ *   0 score-consistency flag | sums over the heads: 1 consistency_violation, 2 boundary_triggered, 3 rung1_triggered,
+ *   4 value_promoted_blocks, 5 dense, 6 exploration_blocks, 7 ranking_disagree_r1, 8 ranking_disagree_r3 |
+ *   k_star: 9 sum, 10 min, 11 max | 12 delta sum | e_val: 13 sum, 14 max | e_pre: 15 sum, 16 max | 17 tau_actual sum |
+ *   tail_mass: 18 sum, 19 max | 20 int8_top1 sum | 21 fp16_top1 sum | fp16_top1 - fp16_top2: 22 sum, 23 min |
+ *   2 exp(2 delta) tail_mass (exp(2 delta) - 1): 24 sum, 25 max | 26 (head, block) pairs outside the FP16-key mask |
+ *   sums of the mass fractions: 27 sum, 28 max | 29 largest eta_b | 30 largest nu_b of the active blocks |
+ *   31 blocks that at least one head reads from the Tier-2 values. */
+#define CQA_SUMMARY_ITEMS 32
+int cqa_step_stats(const cqa_cache *c, const cqa_workspace *ws, int64_t nq, int64_t nact, void *scratch,
+                   double *summary_host, void *stream);
 
 /* Fused append-and-quantise of one token at position `pos` for every KV head:
  * Tier-2 rows, nu_b, per-token INT4 (unless `defer_int4`), and, when the token
