@@ -5,22 +5,26 @@
 //
 // The attend and certifier kernels read a non-resident block straight from the
 // backing array (pinned host memory), so a miss costs bandwidth, never a wait.
-// After the step, three small launches make the next steps faster:
+// After the step, two small launches make the next steps faster:
 //   mark   one thread per block: the block was used if any head has it in the
 //          FP16-key mask (tier 0) / FP16-value mask (tier 1).  Resident ->
 //          stamp its slot with the step number (hit); not resident -> append
-//          to the miss list.
-//   assign one warp per tier walks the slots from the clock hand, takes those
-//          not stamped in this step, evicts their owners and hands them to
-//          the missed blocks (at most max_fill_blocks per call).
+//          to the miss list.  The last CTA then assigns: one warp per tier
+//          walks the slots from the clock hand, takes those not stamped in this
+//          step, evicts their owners and hands them to the missed blocks (at
+//          most max_fill_blocks per call), and closes the step's counters.
 //   fill   one CTA per (assigned block, KV head) copies the 16 rows from the
 //          backing array into the slot.
+// (As a copy of the counters and four launches in a row the update took 16 us
+// of a 32768-token step, most of it between the launches.)
 // Everything is stream-ordered; no kernel waits on another.
 #include "common.cuh"
 
 namespace cqa {
 
-constexpr int HT_STEP = 0, HT_HAND = 1, HT_TIER0 = 3;   // counters layout: [step, hand_k, hand_v, k:{hit,miss,fill,evict}, v:{...}]
+// counters layout: [step, hand_k, hand_v, k:{hit,miss,fill,evict}, v:{...}], one word of open hits (k in the lower half, v in
+// the upper), the values from before the latest update in [12..22], one ticket word.
+constexpr int HT_STEP = 0, HT_HAND = 1, HT_TIER0 = 3, HT_OPEN_HITS = 11, HT_BEFORE = 12, HT_TICKET = 23;
 
 struct HotTierView {
     int32_t *slots, *owner, *stamp, *work;
@@ -40,27 +44,122 @@ __device__ __forceinline__ HotTierView tier_view(const cqa_hot_tier &ht, int tie
     return v;
 }
 
+__device__ __forceinline__ void assign_slots(const cqa_hot_tier &ht, int tier, long max_blocks)
+{
+    const int lane = threadIdx.x & 31;
+    const HotTierView v = tier_view(ht, tier, max_blocks);
+    const int step = (int)ht.counters[HT_STEP];
+    const int cap = tier == 0 ? ht.key_capacity_blocks : ht.value_capacity_blocks;
+    int n_miss = __ldcg(v.work);
+    if (n_miss > ht.max_fill_blocks) n_miss = ht.max_fill_blocks;
+    int hand = (int)(*v.hand % cap);
+    int given = 0;
+    // walk the slots once from the hand, 32 at a time; a slot is free for taking if it was not used in this step
+    for (int base = 0; base < cap && given < n_miss; base += 32) {
+        const int idx = base + lane;
+        int s = hand + idx;
+        if (s >= cap) s -= cap;
+        const bool ok = idx < cap && __ldcg(v.stamp + s) != step;
+        const unsigned who = __ballot_sync(FULL, ok);
+        const int rank = given + __popc(who & ((1u << lane) - 1u));
+        if (ok && rank < n_miss) {
+            const int b = __ldcg(v.work + 2 + rank);
+            const int old = v.owner[s];
+            if (old >= 0) {
+                v.slots[old] = -1;
+                atomicAdd(reinterpret_cast<unsigned long long *>(v.ctr + 3), 1ull);
+            }
+            v.owner[s] = b;
+            v.slots[b] = s;
+            v.stamp[s] = step;
+            v.work[2 + max_blocks + 2 * rank] = b;
+            v.work[2 + max_blocks + 2 * rank + 1] = s;
+        }
+        given += __popc(who);
+        if (given >= n_miss) {
+            // the hand stops behind the last slot taken
+            const int taken_in_chunk = n_miss - (given - __popc(who));
+            int last = -1;
+            unsigned w = who;
+            for (int k = 0; k < taken_in_chunk; ++k) { last = __ffs(w) - 1; w &= w - 1; }
+            hand = hand + base + last + 1;
+        }
+    }
+    if (given > n_miss) given = n_miss;
+    __syncwarp();
+    if (lane == 0) {
+        if (given < n_miss || n_miss == 0) hand = (int)(*v.hand % cap);   // nothing (more) to take: the hand stays
+        *v.hand = hand % cap;
+        v.work[1] = given;
+        v.ctr[2] += given;
+    }
+}
+
+
+// The end of a marking launch: the last of its CTAs (in x and y) sums up the step, assigns slots and opens the next step.
+__device__ __forceinline__ void close_marking(const cqa_hot_tier &ht, long max_blocks)
+{
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long *ticket = reinterpret_cast<unsigned long long *>(ht.counters + HT_TICKET);
+        s_last = atomicAdd(ticket, 1ull) == (unsigned long long)gridDim.x * gridDim.y - 1ull;
+        if (s_last) {
+            __threadfence();
+            // the counters before this update, for callers that report per-call figures; then its hits and misses
+            for (int i = 0; i < HT_OPEN_HITS; ++i) ht.counters[HT_BEFORE + i] = ht.counters[i];
+            const unsigned long long hits = __ldcg(reinterpret_cast<unsigned long long *>(ht.counters + HT_OPEN_HITS));
+            for (int tier = 0; tier < 2; ++tier) {
+                const HotTierView v = tier_view(ht, tier, max_blocks);
+                v.ctr[0] += (int64_t)(tier == 0 ? hits & 0xFFFFFFFFull : hits >> 32);
+                v.ctr[1] += __ldcg(v.work);
+            }
+            ht.counters[HT_OPEN_HITS] = 0;
+            *ticket = 0;
+            __threadfence_block();
+        }
+    }
+    __syncthreads();
+    if (!s_last) return;
+    if (threadIdx.x < 64) assign_slots(ht, threadIdx.x >> 5, max_blocks);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ht.counters[HT_STEP] += 1;
+        for (int tier = 0; tier < 2; ++tier) tier_view(ht, tier, max_blocks).work[0] = 0;
+    }
+}
+
+// Stamps the slot of a used block, or lists the block as missing.
+__device__ __forceinline__ void mark_block(const cqa_hot_tier &ht, int tier, long b, bool used, long max_blocks)
+{
+    const HotTierView v = tier_view(ht, tier, max_blocks);
+    const int s = used ? v.slots[b] : -1;
+    if (used && s >= 0) {
+        v.stamp[s] = (int)ht.counters[HT_STEP];
+    } else if (used) {
+        const int i = atomicAdd(v.work + 0, 1);
+        v.work[2 + i] = (int)b;
+    }
+    const unsigned hits = __popc(__ballot_sync(FULL, used && s >= 0));
+    if ((threadIdx.x & 31) == 0 && hits)
+        atomicAdd(reinterpret_cast<unsigned long long *>(ht.counters + HT_OPEN_HITS), (unsigned long long)hits << (32 * tier));
+}
+
 __global__ void __launch_bounds__(256) hot_mark_kernel(cqa_hot_tier ht, cqa_workspace ws, int n_heads, long nact,
                                                       long max_blocks)
 {
     const int tier = blockIdx.y;
-    const HotTierView v = tier_view(ht, tier, max_blocks);
+    grid_dependency_wait();
     const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nact) return;
-    const unsigned char *mask = tier == 0 ? ws.topk_mask : ws.value_mask;
-    bool used = false;
-    for (int h = 0; h < n_heads; ++h) used |= mask[(long)h * ws.ld + b] != 0;
-    if (!used) return;
-    const int step = (int)ht.counters[HT_STEP];
-    const int s = v.slots[b];
-    if (s >= 0) {
-        v.stamp[s] = step;
-        atomicAdd(reinterpret_cast<unsigned long long *>(v.ctr + 0), 1ull);
-    } else {
-        const int i = atomicAdd(v.work + 0, 1);
-        v.work[2 + i] = (int)b;
-        atomicAdd(reinterpret_cast<unsigned long long *>(v.ctr + 1), 1ull);
+    int used = 0;
+    if (b < nact) {
+        const unsigned char *mask = tier == 0 ? ws.topk_mask : ws.value_mask;
+#pragma unroll 16
+        for (int h = 0; h < n_heads; ++h) used |= mask[(long)h * ws.ld + b];
     }
+    mark_block(ht, tier, b, used != 0, max_blocks);
+    close_marking(ht, max_blocks);
 }
 
 // The same marking for an explicit list of block ids of one tier (a caller that knows which blocks it is about to
@@ -68,21 +167,10 @@ __global__ void __launch_bounds__(256) hot_mark_kernel(cqa_hot_tier ht, cqa_work
 __global__ void __launch_bounds__(256) hot_mark_list_kernel(cqa_hot_tier ht, int tier, const int64_t *blocks, long n,
                                                            long max_blocks)
 {
-    const HotTierView v = tier_view(ht, tier, max_blocks);
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const long b = blocks[i];
-    if (b < 0 || b >= max_blocks) return;
-    const int step = (int)ht.counters[HT_STEP];
-    const int s = v.slots[b];
-    if (s >= 0) {
-        v.stamp[s] = step;
-        atomicAdd(reinterpret_cast<unsigned long long *>(v.ctr + 0), 1ull);
-    } else {
-        const int k = atomicAdd(v.work + 0, 1);
-        v.work[2 + k] = (int)b;
-        atomicAdd(reinterpret_cast<unsigned long long *>(v.ctr + 1), 1ull);
-    }
+    const long b = i < n ? blocks[i] : -1;
+    mark_block(ht, tier, b, b >= 0 && b < max_blocks, max_blocks);
+    close_marking(ht, max_blocks);
 }
 
 // Gather of 16-row blocks from a backing array (row = token index) into the slots of a scratch array, 16 bytes per
@@ -125,61 +213,11 @@ __global__ void __launch_bounds__(256) slot_table_update_kernel(const int64_t *l
     }
 }
 
-__global__ void __launch_bounds__(32) hot_assign_kernel(cqa_hot_tier ht, long max_blocks)
-{
-    const int tier = blockIdx.x, lane = threadIdx.x;
-    const HotTierView v = tier_view(ht, tier, max_blocks);
-    const int step = (int)ht.counters[HT_STEP];
-    const int cap = tier == 0 ? ht.key_capacity_blocks : ht.value_capacity_blocks;
-    int n_miss = v.work[0];
-    if (n_miss > ht.max_fill_blocks) n_miss = ht.max_fill_blocks;
-    int hand = (int)(*v.hand % cap);
-    int given = 0;
-    // walk the slots once from the hand, 32 at a time; a slot is free for taking if it was not used in this step
-    for (int base = 0; base < cap && given < n_miss; base += 32) {
-        const int idx = base + lane;
-        int s = hand + idx;
-        if (s >= cap) s -= cap;
-        const bool ok = idx < cap && v.stamp[s] != step;
-        const unsigned who = __ballot_sync(FULL, ok);
-        const int rank = given + __popc(who & ((1u << lane) - 1u));
-        if (ok && rank < n_miss) {
-            const int b = v.work[2 + rank];
-            const int old = v.owner[s];
-            if (old >= 0) {
-                v.slots[old] = -1;
-                atomicAdd(reinterpret_cast<unsigned long long *>(v.ctr + 3), 1ull);
-            }
-            v.owner[s] = b;
-            v.slots[b] = s;
-            v.stamp[s] = step;
-            v.work[2 + max_blocks + 2 * rank] = b;
-            v.work[2 + max_blocks + 2 * rank + 1] = s;
-        }
-        given += __popc(who);
-        if (given >= n_miss) {
-            // the hand stops behind the last slot taken
-            const int taken_in_chunk = n_miss - (given - __popc(who));
-            int last = -1;
-            unsigned w = who;
-            for (int k = 0; k < taken_in_chunk; ++k) { last = __ffs(w) - 1; w &= w - 1; }
-            hand = hand + base + last + 1;
-        }
-    }
-    if (given > n_miss) given = n_miss;
-    __syncwarp();
-    if (lane == 0) {
-        if (given < n_miss || n_miss == 0) hand = (int)(*v.hand % cap);   // nothing (more) to take: the hand stays
-        *v.hand = hand % cap;
-        v.work[1] = given;
-        v.ctr[2] += given;
-    }
-}
-
 template <typename T2>
 __global__ void __launch_bounds__(128) hot_fill_kernel(cqa_hot_tier ht, cqa_cache c, long max_blocks)
 {
     const int tier = blockIdx.z, kv = blockIdx.y, i = blockIdx.x;
+    grid_dependency_wait();
     const HotTierView v = tier_view(ht, tier, max_blocks);
     if (i >= v.work[1]) return;
     const long b = v.work[2 + max_blocks + 2 * i], s = v.work[2 + max_blocks + 2 * i + 1];
@@ -191,19 +229,6 @@ __global__ void __launch_bounds__(128) hot_fill_kernel(cqa_hot_tier ht, cqa_cach
     uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<T2 *>(hot) + ((long)kv * hot_rows + s * BS) * D);
     constexpr int N16 = BS * D * (int)sizeof(T2) / 16;
     for (int k = threadIdx.x; k < N16; k += 128) dst[k] = src[k];
-}
-
-__global__ void hot_finish_kernel(cqa_hot_tier ht, long max_blocks)
-{
-    // next step; clear the per-step lists
-    if (threadIdx.x == 0) {
-        ht.counters[HT_STEP] += 1;
-        for (int tier = 0; tier < 2; ++tier) {
-            int32_t *w = ht.work + (long)tier * (2 + 3 * max_blocks);
-            w[0] = 0;
-            w[1] = 0;
-        }
-    }
 }
 
 }  // namespace cqa
@@ -232,13 +257,13 @@ static int check_hot_tier(const cqa_cache *c, const cqa_hot_tier *ht, const char
     return CQA_OK;
 }
 
-static void launch_fill(const cqa_cache *c, const cqa_hot_tier *ht, cudaStream_t st)
+static int launch_fill(const cqa_cache *c, const cqa_hot_tier *ht, cudaStream_t st)
 {
     dim3 gf((unsigned)ht->max_fill_blocks, (unsigned)c->kv_heads, 2);
     switch (c->t2_dtype) {
-    case CQA_F32: hot_fill_kernel<float><<<gf, 128, 0, st>>>(*ht, *c, c->max_blocks); note_launch(); break;
-    case CQA_F16: hot_fill_kernel<__half><<<gf, 128, 0, st>>>(*ht, *c, c->max_blocks); note_launch(); break;
-    default: hot_fill_kernel<__nv_bfloat16><<<gf, 128, 0, st>>>(*ht, *c, c->max_blocks); note_launch(); break;
+    case CQA_F32: return check_cuda(launch_chained(hot_fill_kernel<float>, gf, dim3(128), 0, st, true, *ht, *c, (long)c->max_blocks), "hot_fill_kernel");
+    case CQA_F16: return check_cuda(launch_chained(hot_fill_kernel<__half>, gf, dim3(128), 0, st, true, *ht, *c, (long)c->max_blocks), "hot_fill_kernel");
+    default: return check_cuda(launch_chained(hot_fill_kernel<__nv_bfloat16>, gf, dim3(128), 0, st, true, *ht, *c, (long)c->max_blocks), "hot_fill_kernel");
     }
 }
 
@@ -251,16 +276,10 @@ extern "C" int cqa_hot_tier_ensure(const cqa_cache *c, const cqa_hot_tier *ht, i
     const int rc = check_hot_tier(c, ht, "cqa_hot_tier_ensure");
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    // the counters before this call, for callers that report per-call figures
-    cudaMemcpyAsync(ht->counters + 12, ht->counters, 12 * sizeof(int64_t), cudaMemcpyDeviceToDevice, st);
-    if (n > 0) {
-        hot_mark_list_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(*ht, tier, block_ids, n, c->max_blocks);
-        note_launch();
-    }
-    hot_assign_kernel<<<2, 32, 0, st>>>(*ht, c->max_blocks); note_launch();
-    launch_fill(c, ht, st);
-    hot_finish_kernel<<<1, 32, 0, st>>>(*ht, c->max_blocks); note_launch();
-    return check_launch("hot tier kernels");
+    const unsigned ctas = n > 0 ? (unsigned)((n + 255) / 256) : 1u;
+    const int rc2 = check_cuda(launch_chained(hot_mark_list_kernel, dim3(ctas), dim3(256), 0, st, false, *ht, tier, block_ids, (long)n,
+                                              (long)c->max_blocks), "hot_mark_list_kernel");
+    return rc2 ? rc2 : launch_fill(c, ht, st);
 }
 
 static const char *device_view(const void *p)
@@ -342,12 +361,8 @@ extern "C" int cqa_hot_tier_update(const cqa_cache *c, const cqa_workspace *ws, 
     if (c->t2_dtype < 0 || c->t2_dtype > 2) { set_error("cqa_hot_tier_update: unknown Tier-2 dtype"); return CQA_ERR_INVALID; }
     cudaStream_t st = (cudaStream_t)stream;
     const int H = c->kv_heads * c->gqa_group;
-    // counters[12..23] keep the values from before this step, so the host can report per-step figures
-    cudaMemcpyAsync(ht->counters + 12, ht->counters, 12 * sizeof(int64_t), cudaMemcpyDeviceToDevice, st);
     dim3 gm((unsigned)((nact + 255) / 256), 2);
-    hot_mark_kernel<<<gm, 256, 0, st>>>(*ht, *ws, H, nact, c->max_blocks); note_launch();
-    hot_assign_kernel<<<2, 32, 0, st>>>(*ht, c->max_blocks); note_launch();
-    launch_fill(c, ht, st);
-    hot_finish_kernel<<<1, 32, 0, st>>>(*ht, c->max_blocks); note_launch();
-    return check_launch("hot tier kernels");
+    const int rc = check_cuda(launch_chained(hot_mark_kernel, gm, dim3(256), 0, st, true, *ht, *ws, H, (long)nact, (long)c->max_blocks),
+                              "hot_mark_kernel");
+    return rc ? rc : launch_fill(c, ht, st);
 }

@@ -19,6 +19,7 @@ replacement and counters live on the device (csrc/hot_tier.cu).
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from collections import OrderedDict
 from collections.abc import Mapping
 from dataclasses import dataclass, field
@@ -30,6 +31,10 @@ from cqa_b200 import _lib
 
 BLOCK = 16
 HEAD_DIM = 128
+
+_DESC_LAYOUT = struct.Struct("4i2q12Q1Q1q1Q1q4Q1q")             # _lib.CqaCache
+_ITEM_LAYOUT = struct.Struct("2Q2q2i")                            # _lib.CqaPrefillItem behind its cache
+assert _DESC_LAYOUT.size == C.sizeof(_lib.CqaCache) and _DESC_LAYOUT.size + _ITEM_LAYOUT.size == C.sizeof(_lib.CqaPrefillItem)
 
 # the current device and its current stream without torch's checks (a CUDA tensor at hand means CUDA is initialised)
 _get_device = getattr(torch._C, "_cuda_getDevice", None)
@@ -125,39 +130,23 @@ class TieredKeyCacheLayer:
         cached = self._desc_cache.get(g)
         if cached is not None:
             return cached
-        d = _lib.CqaCache()
-        d.kv_heads = self.kv_heads
-        d.gqa_group = g
-        t2 = self.keys_fp16_gpu
-        d.t2_dtype = _lib.dtype_code(t2.dtype) if t2 is not None else _lib.CQA_F16
-        d.cap_tokens = int(self.keys_int8.shape[1])
-        d.max_blocks = int(self.keys_scale.shape[1])
-        d.keys_int8 = _lib.ptr(self.keys_int8)
-        d.keys_scale = _lib.ptr(self.keys_scale)
-        d.keys_zero_points = _lib.ptr(self.keys_zero_points)
-        d.correction = _lib.ptr(self.correction)
-        d.sigma_max = _lib.ptr(self.keys_scale_max)
-        d.values_int4_packed = _lib.ptr(self.values_int4_packed)
-        d.values_int4_scales = _lib.ptr(self.values_int4_scales)
-        d.values_int4_zeros = _lib.ptr(self.values_int4_zeros)
-        d.values_int4_errors = _lib.ptr(self.values_int4_errors)
-        d.values_int4_error_sums = _lib.ptr(self.values_int4_error_sums)
-        d.values_int4_error_counts = _lib.ptr(self.values_int4_error_counts)
-        d.values_norm_max = _lib.ptr(self.values_norm_max_per_block)
-        d.keys_t2 = _lib.ptr(t2)
-        d.keys_t2_rows = int(t2.shape[1]) if t2 is not None else 0
+        p = _lib.ptr
+        kt2 = self.keys_fp16_gpu
         vt2 = self.values_fp16 if self.values_fp16 is not None else self.values_fp16_gpu
-        d.values_t2 = _lib.ptr(vt2)
-        d.values_t2_rows = int(vt2.shape[1]) if vt2 is not None else 0
-        d.key_slots = None      # identity: full mirrors
-        d.value_slots = None
+        slots = (0, 0, 0, 0, 0)      # identity: full mirrors
         if self._hot is not None:
             # bounded hot tier: the *_gpu arrays are slot scratch, the pinned *_cpu arrays back them
-            d.key_slots = self._hot["key_slots"].data_ptr()
-            d.value_slots = self._hot["value_slots"].data_ptr()
-            d.keys_t2_backing = self.keys_fp16_cpu.data_ptr()
-            d.values_t2_backing = self.values_fp16_cpu.data_ptr()
-            d.t2_backing_rows = int(self.keys_fp16_cpu.shape[1])
+            slots = (self._hot["key_slots"].data_ptr(), self._hot["value_slots"].data_ptr(), self.keys_fp16_cpu.data_ptr(),
+                     self.values_fp16_cpu.data_ptr(), int(self.keys_fp16_cpu.shape[1]))
+        # in the order of the struct's fields, packed at once (a third of the time of setting them one by one)
+        d = _lib.CqaCache.from_buffer_copy(_DESC_LAYOUT.pack(
+            self.kv_heads, g, _lib.dtype_code(kt2.dtype) if kt2 is not None else _lib.CQA_F16, 0,
+            self.keys_int8.shape[1], self.keys_scale.shape[1],
+            p(self.keys_int8) or 0, p(self.keys_scale) or 0, p(self.keys_zero_points) or 0, p(self.correction) or 0,
+            p(self.keys_scale_max) or 0, p(self.values_int4_packed) or 0, p(self.values_int4_scales) or 0,
+            p(self.values_int4_zeros) or 0, p(self.values_int4_errors) or 0, p(self.values_int4_error_sums) or 0,
+            p(self.values_int4_error_counts) or 0, p(self.values_norm_max_per_block) or 0,
+            p(kt2) or 0, kt2.shape[1] if kt2 is not None else 0, p(vt2) or 0, vt2.shape[1] if vt2 is not None else 0, *slots))
         self._desc_cache[g] = d
         return d
 
@@ -176,9 +165,10 @@ class TieredKeyCacheLayer:
     @classmethod
     def _allocate(cls, keys: torch.Tensor, values: torch.Tensor, block_size: int, max_pagein_blocks: int,
                   max_new_tokens: int, int4: bool, group_size: int, hot_blocks: tuple[int, int] | None = None,
-                  sigma_max: torch.Tensor | None = None) -> "TieredKeyCacheLayer":
-        """The cache's arrays.  A full mirror's are left uninitialised: the encode that follows writes the prompt and
-        sets the capacity behind it to the empty state (`init_reserve`), one launch in place of a fill per array."""
+                  sigma_max: torch.Tensor | None = None, tokens: int | None = None) -> "TieredKeyCacheLayer":
+        """The cache's arrays, for `tokens` of the given keys (all of them by default).  A full mirror's are left
+        uninitialised: the encode that follows writes the prompt and sets the capacity behind it to the empty state
+        (`init_reserve`), one launch in place of a fill per array."""
         _require_cuda(keys, "keys")
         _require_cuda(values, "values")
         if block_size != BLOCK:
@@ -186,13 +176,13 @@ class TieredKeyCacheLayer:
         if int4 and group_size != 16:
             raise ValueError("INT4 group_size must be 16 (fixed by the kernels)")
         kv, N, hd = keys.shape
+        if tokens is not None:
+            N = tokens
         dv = values.shape[2]
         if hd != HEAD_DIM or dv != HEAD_DIM:
             raise ValueError(f"head_dim and d_v must be 128 (got {hd}, {dv})")
         if N % BLOCK != 0:
             raise ValueError("N must be block aligned; append the remainder with append_token")
-        if keys.dtype != values.dtype:
-            values = values.to(keys.dtype)
         _lib.dtype_code(keys.dtype)
         dev = keys.device
         nb = N // BLOCK
@@ -269,11 +259,11 @@ class TieredKeyCacheLayer:
     def from_fp16_cache(cls, keys_fp16: torch.Tensor, values_fp16: torch.Tensor, block_size: int = 16,
                         max_pagein_blocks: int = 64, max_new_tokens: int = 512,
                         fp16_key_cache_capacity: int | None = None, _encode: bool = True,
-                        _sigma_max: torch.Tensor | None = None) -> "TieredKeyCacheLayer":
+                        _sigma_max: torch.Tensor | None = None, _tokens: int | None = None) -> "TieredKeyCacheLayer":
         """INT8 keys + model-dtype values (reference: tiered_kv_cache.py:135-286).  `_encode=False` only allocates
         (the whole-model constructors encode every layer in one library call afterwards)."""
         self = cls._allocate(keys_fp16, values_fp16, block_size, max_pagein_blocks, max_new_tokens,
-                             int4=False, group_size=16, sigma_max=_sigma_max)
+                             int4=False, group_size=16, sigma_max=_sigma_max, tokens=_tokens)
         cap = cls._check_capacity(fp16_key_cache_capacity, self.keys_scale.shape[1], "fp16_key_cache_capacity")
         if cap is not None and cap < self.keys_scale.shape[1]:
             raise NotImplementedError(
@@ -293,9 +283,10 @@ class TieredKeyCacheLayer:
                               fp16_key_cache_capacity: int | None = None,
                               fp16_value_cache_capacity: int | None = None,
                               defer_int4_append_quantization: bool = False,
-                              _encode: bool = True, _sigma_max: torch.Tensor | None = None) -> "TieredKeyCacheLayer":
+                              _encode: bool = True, _sigma_max: torch.Tensor | None = None,
+                              _tokens: int | None = None) -> "TieredKeyCacheLayer":
         """INT8 keys + INT4 g16 values (reference: tiered_kv_cache.py:289-405).  `_encode=False` only allocates."""
-        nb0 = keys_fp16.shape[1] // BLOCK
+        nb0 = (keys_fp16.shape[1] if _tokens is None else _tokens) // BLOCK
         maxblk = nb0 + (max_new_tokens + BLOCK - 1) // BLOCK
         kcap = cls._check_capacity(fp16_key_cache_capacity, maxblk, "fp16_key_cache_capacity")
         vcap = cls._check_capacity(fp16_value_cache_capacity, maxblk, "fp16_value_cache_capacity")
@@ -307,7 +298,8 @@ class TieredKeyCacheLayer:
             hot_blocks = (min(kcap, maxblk) if kcap is not None else maxblk,
                           min(vcap, maxblk) if vcap is not None else maxblk)
         self = cls._allocate(keys_fp16, values_fp16, block_size, max_pagein_blocks, max_new_tokens,
-                             int4=True, group_size=group_size, hot_blocks=hot_blocks, sigma_max=_sigma_max)
+                             int4=True, group_size=group_size, hot_blocks=hot_blocks, sigma_max=_sigma_max,
+                             tokens=_tokens)
         if bounded:
             self.defer_int4_append_quantization = bool(defer_int4_append_quantization)
             if _encode:
@@ -566,13 +558,12 @@ def _layer_kv(past_kv, layer_id: int, batch_index: int = 0):
     return past_kv[layer_id][0][batch_index], past_kv[layer_id][1][batch_index]
 
 
-def _layer_sigma_max(past_kv, layer_ids: list, batch_index: int = 0):
+def _sigma_max_rows(layers):
     """The layers' running channel maxima, zeroed by one fill (None per layer when the layers differ in heads or device)."""
-    shapes = {(k.shape[0], k.shape[2], k.device) for k in (_layer_kv(past_kv, l, batch_index)[0] for l in layer_ids)}
-    if len(shapes) != 1:
-        return [None] * len(layer_ids)
-    kv, hd, dev = shapes.pop()
-    return torch.zeros(len(layer_ids), kv, hd, dtype=torch.float32, device=dev).unbind(0)
+    k0 = layers[0][0] if layers else None
+    if any(k.shape[0] != k0.shape[0] or k.device != k0.device for k, _ in layers[1:]) or not layers:
+        return [None] * len(layers)
+    return torch.zeros(len(layers), k0.shape[0], k0.shape[2], dtype=torch.float32, device=k0.device).unbind(0)
 
 
 def _encode_prefill_layers(entries) -> None:
@@ -586,25 +577,21 @@ def _encode_prefill_layers(entries) -> None:
             values = values.to(keys.dtype)
         # rows of 128 contiguous elements with one row stride per KV head are read in place (a slice of a longer
         # [KV, rows, 128] buffer, as HF caches hand out); anything else is copied once
-        def row_stride(t):
-            ok = t.stride(2) == 1 and t.stride(1) == HEAD_DIM and t.stride(0) % HEAD_DIM == 0
-            return t.stride(0) // HEAD_DIM if ok and t.stride(0) >= t.shape[1] * HEAD_DIM else None
-        rk, rv = row_stride(keys), row_stride(values)
-        if rk is None or rk != rv:
+        s0, s1, s2 = keys.stride()
+        if s2 != 1 or s1 != HEAD_DIM or s0 % HEAD_DIM or s0 < seq_len * HEAD_DIM or values.stride() != (s0, s1, s2):
             keys, values = keys.contiguous(), values.contiguous()
-            rk = keys.shape[1]
+            s0 = keys.shape[1] * HEAD_DIM
+        rk = s0 // HEAD_DIM
         groups.setdefault((keys.device, keys.dtype), []).append((cache, keys, values, seq_len, rk))
     for (dev, dtype), group in groups.items():
-        items = (_lib.CqaPrefillItem * len(group))()
-        for i, (cache, keys, values, seq_len, rows) in enumerate(group):
-            items[i].cache = cache._desc()
+        records = bytearray()
+        for cache, keys, values, seq_len, rows in group:
             # an empty prompt has no memory of its own; nothing is read from it
-            items[i].k_src = keys.data_ptr() or cache.keys_int8.data_ptr()
-            items[i].v_src = values.data_ptr() or cache.keys_int8.data_ptr()
-            items[i].src_rows = rows
-            items[i].init_reserve = 0 if cache.bounded_hot_tier else 1
-            items[i].n_tokens = seq_len
-            items[i].defer_int4 = 1 if cache._defer_int4_flag() else 0
+            spare = cache.keys_int8.data_ptr()
+            records += bytes(cache._desc())
+            records += _ITEM_LAYOUT.pack(keys.data_ptr() or spare, values.data_ptr() or spare, rows, seq_len,
+                                         1 if cache._defer_int4_flag() else 0, 0 if cache.bounded_hot_tier else 1)
+        items = (_lib.CqaPrefillItem * len(group)).from_buffer(records)
         with _lib.on_device(dev):
             rc = _lib.lib().cqa_prefill_encode(items, len(group), _lib.dtype_code(dtype), _lib.current_stream(dev))
         _lib.check(rc, "cqa_prefill_encode")
@@ -626,18 +613,17 @@ def create_tiered_cache_int4v_from_model(past_kv, layer_ids: list, block_size: i
     if defer_int4_append_quantization is None:
         defer_int4_append_quantization = fp16_value_cache_capacity is None
     caches, entries = {}, []
-    sigma = _layer_sigma_max(past_kv, layer_ids, batch_index)
-    for layer_id, sigma_max in zip(layer_ids, sigma):
-        keys, values = _layer_kv(past_kv, layer_id, batch_index)
+    layers = [_layer_kv(past_kv, layer_id, batch_index) for layer_id in layer_ids]
+    for layer_id, (keys, values), sigma_max in zip(layer_ids, layers, _sigma_max_rows(layers)):
         seq_len = keys.shape[1]
         aligned = (seq_len // block_size) * block_size
         cache = TieredKeyCacheLayer.from_fp16_cache_int4v(
-            keys[:, :aligned, :], values[:, :aligned, :],
-            block_size=block_size, group_size=group_size,
+            keys, values, block_size=block_size, group_size=group_size,
             max_new_tokens=max_new_tokens + (seq_len - aligned),
             fp16_key_cache_capacity=fp16_key_cache_capacity,
             fp16_value_cache_capacity=fp16_value_cache_capacity,
             defer_int4_append_quantization=bool(defer_int4_append_quantization), _encode=False, _sigma_max=sigma_max,
+            _tokens=aligned,
         )
         cache.num_tokens = cache.num_blocks = cache.num_quantized_blocks = 0
         entries.append((cache, keys, values, seq_len))
@@ -650,15 +636,13 @@ def create_tiered_cache_from_model(past_kv, layer_ids: list, block_size: int = 1
                                    fp16_key_cache_capacity: int | None = None) -> dict:
     """Per-layer INT8-key / model-dtype-value caches (reference: tiered_kv_cache.py:1644-1701)."""
     caches, entries = {}, []
-    sigma = _layer_sigma_max(past_kv, layer_ids)
-    for layer_id, sigma_max in zip(layer_ids, sigma):
-        keys, values = _layer_kv(past_kv, layer_id)
+    layers = [_layer_kv(past_kv, layer_id) for layer_id in layer_ids]
+    for layer_id, (keys, values), sigma_max in zip(layer_ids, layers, _sigma_max_rows(layers)):
         seq_len = keys.shape[1]
         aligned = (seq_len // block_size) * block_size
         cache = TieredKeyCacheLayer.from_fp16_cache(
-            keys[:, :aligned, :], values[:, :aligned, :],
-            block_size=block_size, max_new_tokens=max_new_tokens + (seq_len - aligned),
-            fp16_key_cache_capacity=fp16_key_cache_capacity, _encode=False, _sigma_max=sigma_max,
+            keys, values, block_size=block_size, max_new_tokens=max_new_tokens + (seq_len - aligned),
+            fp16_key_cache_capacity=fp16_key_cache_capacity, _encode=False, _sigma_max=sigma_max, _tokens=aligned,
         )
         cache.num_tokens = cache.num_blocks = cache.num_quantized_blocks = 0
         entries.append((cache, keys, values, seq_len))
