@@ -547,7 +547,8 @@ typedef struct cqa_hot_tier {
     int32_t *value_stamp;
     int32_t *work;               /* [2][2 + 3 * max_blocks] per tier: miss count, fill count, missed blocks, (block, slot) pairs */
     int64_t *counters;           /* [24]: step, clock hands (keys, values), then per tier: hits, misses, page-ins, evictions;
-                                    1 spare; entries 12..23 repeat 0..11 as they were before the latest update call */
+                                    entries 12..22 repeat 0..10 as they were before the latest update call;
+                                    11 and 23 belong to the update and are 0 between calls */
 } cqa_hot_tier;
 
 int cqa_hot_tier_update(const cqa_cache *c, const cqa_workspace *ws, const cqa_hot_tier *ht, int64_t nact,
