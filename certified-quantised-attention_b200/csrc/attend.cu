@@ -8,9 +8,9 @@
 //     measured the same.)  Softmax weights are made in the layout of the matrix products' B fragments.
 //   * (head, block) pairs flagged in topk_mask take their logits from Tier-2 keys, pairs flagged in value_mask their
 //     values from Tier 2: the same products, the four heads together.  The rows are requested into L2 two pairs ahead.
-//   * Heads that the certificate flags for the dense FP16 recompute: when a CTA is done with its split it takes units
-//     of (group with a flagged head, chunk of blocks); CTAs beyond the splits, where the GPU has room for them, start
-//     there.  With no flagged head this is one word read.
+//   * Heads that the certificate flags for the dense FP16 recompute: when a CTA is done with its split it draws units
+//     of (group with a flagged head, chunk of blocks) from a counter; CTAs beyond the splits, where the GPU has room for
+//     them, start there.  With no flagged head this is one word read.
 //   * The last CTA to finish for a KV head (a group, for the dense part) merges the split partials and writes the
 //     output rows; no separate merge launch.
 //
@@ -608,8 +608,8 @@ __device__ __forceinline__ void cta_merge_store(const float *sm_m, const float *
 // Final merge of `ns` split partials of heads [head0, head0+nh) by the last CTA to arrive.
 // All 256 threads take part; `sm` is 16-byte aligned scratch of at least 2*nh*ns + nh + 3 + 8*128 floats.
 // A thread owns one float4 column of one head and every (256 / (32*nh))-th split.  Its accumulator rows are
-// requested first (up to 20 loads in flight per thread), then the (m, l) partials go through shared memory and
-// one warp per head turns them into per-split scales while those loads are still travelling; the rows are then
+// requested first (up to 20 loads in flight per thread) together with the (m, l) partials, which go through shared
+// memory and which one warp per head turns into per-split scales; the rows are then
 // scaled and summed, the per-thread sums combined through shared memory, normalised and written.
 __device__ __forceinline__ void final_merge(const float *pm, const float *pl, const float *pa, int ns, int head0,
                                             int nh, const cqa_workspace &ws, bool dense_role, float *sm, int kv_heads, int n_heads_total,
@@ -624,13 +624,19 @@ __device__ __forceinline__ void final_merge(const float *pm, const float *pl, co
     const int g = warp / nparts, part = warp % nparts;
     const float4 *rows = reinterpret_cast<const float4 *>(pa + (long)(head0 + g) * ns * D) + lane;
     float4 buf[BATCH];
+    const auto load_rows = [&](int first) {
 #pragma unroll
-    for (int j = 0; j < BATCH; ++j) {
-        const int sp = part + j * nparts;
-        buf[j] = sp < ns ? __ldcg(rows + (long)sp * (D / 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
+        for (int j = 0; j < BATCH; ++j) {
+            const int sp = first + part + j * nparts;
+            buf[j] = sp < ns ? __ldcg(rows + (long)sp * (D / 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    float m_first = 0.0f, l_first = 0.0f;
+    if (tid < nh * ns) { m_first = __ldcg(pm + (long)head0 * ns + tid); l_first = __ldcg(pl + (long)head0 * ns + tid); }
+    load_rows(0);
     __syncthreads();   // the scratch may still be in use as merge buffers
-    for (int i = tid; i < nh * ns; i += ATT_THREADS) {
+    if (tid < nh * ns) { s_m[tid] = m_first; s_sc[tid] = l_first; }
+    for (int i = tid + ATT_THREADS; i < nh * ns; i += ATT_THREADS) {
         s_m[i] = __ldcg(pm + (long)head0 * ns + i);
         s_sc[i] = __ldcg(pl + (long)head0 * ns + i);
     }
@@ -668,25 +674,20 @@ __device__ __forceinline__ void final_merge(const float *pm, const float *pl, co
     }
     __syncthreads();
     float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+    for (int first = 0; first < ns; first += BATCH * nparts) {
+        if (first > 0) load_rows(first);            // more splits than one batch covers
 #pragma unroll
-    for (int j = 0; j < BATCH; ++j) {
-        const int sp = part + j * nparts;
-        if (sp < ns) {
-            const float sc = s_sc[g * ns + sp];
-            a.x = fmaf(buf[j].x, sc, a.x);
-            a.y = fmaf(buf[j].y, sc, a.y);
-            a.z = fmaf(buf[j].z, sc, a.z);
-            a.w = fmaf(buf[j].w, sc, a.w);
+        for (int j = 0; j < BATCH; ++j) {
+            const int sp = first + part + j * nparts;
+            if (sp < ns) {
+                const float sc = s_sc[g * ns + sp];
+                a.x = fmaf(buf[j].x, sc, a.x);
+                a.y = fmaf(buf[j].y, sc, a.y);
+                a.z = fmaf(buf[j].z, sc, a.z);
+                a.w = fmaf(buf[j].w, sc, a.w);
+            }
         }
-    }
-#pragma unroll 4
-    for (int sp = part + BATCH * nparts; sp < ns; sp += nparts) {   // more splits than one batch covers
-        const float4 v = __ldcg(rows + (long)sp * (D / 4));
-        const float sc = s_sc[g * ns + sp];
-        a.x = fmaf(v.x, sc, a.x);
-        a.y = fmaf(v.y, sc, a.y);
-        a.z = fmaf(v.z, sc, a.z);
-        a.w = fmaf(v.w, sc, a.w);
     }
     reinterpret_cast<float4 *>(s_part + warp * D)[lane] = a;
     __syncthreads();
@@ -725,20 +726,21 @@ __device__ __forceinline__ void final_merge(const float *pm, const float *pl, co
     }
 }
 
-// Returns true in every thread of the CTA that took the last ticket.
-__device__ __forceinline__ bool take_ticket(int *ticket, int total, int *s_flag)
+// Returns true in every thread of the CTA that took the last ticket (the bits of `mask` count them).
+__device__ __forceinline__ bool take_ticket(int *ticket, int total, int *s_flag, int mask = -1)
 {
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        const int t = atomicAdd(ticket, 1);
-        *s_flag = (t == total - 1) ? 1 : 0;
-        if (t == total - 1) *ticket = 0;  // ready for the next launch
+        __threadfence();                  // the barrier before it orders the CTA's partials
+        const int last = (atomicAdd(ticket, 1) & mask) == total - 1 ? 1 : 0;
+        if (last) {
+            atomicSub(ticket, total);     // ready for the next launch
+            __threadfence();
+        }
+        *s_flag = last;
     }
     __syncthreads();
-    const bool last = *s_flag != 0;
-    if (last) __threadfence();
-    return last;
+    return *s_flag != 0;
 }
 
 template <typename T2>
@@ -975,14 +977,22 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
     }
     if (n_dense == 0) return;
 
-    // ---- dense recompute of the flagged heads: units of (group of heads with a flagged one, chunk of blocks), dealt to
-    // the CTAs without a split first; the heads of a group share the rows.
+    // ---- dense recompute of the flagged heads: units of (group of heads with a flagged one, chunk of blocks); the heads
+    // of a group share the rows.  A CTA draws its next unit from a counter when it is done with the last one (the splits
+    // end far apart where their promotions differ, and the CTAs that merge come later still; dealt out by CTA number a step
+    // of 8192 tokens fp32 took 69.7 us in place of 64.2, four sequences of 65536 tokens 402 in place of 375).  The counter is the upper 24 bits of the first group's ticket
+    // word: each CTA draws one number past the last unit, and the one with the largest sets it back.
     constexpr int WINDOW = 256;          // groups looked at together
     __shared__ unsigned char s_group[WINDOW], s_heads[WINDOW];
-    __shared__ int s_count;
-    const int groups = c.kv_heads * SUBS, ds = ws.dense_splits, gx = (int)gridDim.x, spare = gx - ns;
-    const int n_ctas = gx * groups;
-    const int id = (split >= ns ? split - ns : spare + split) * groups + (int)blockIdx.y;
+    __shared__ int s_count, s_unit;
+    const int groups = c.kv_heads * SUBS, ds = ws.dense_splits;
+    const int n_ctas = (int)gridDim.x * groups;
+    int *counter = ws.tickets + c.kv_heads;
+    constexpr int UNIT_SHIFT = 8;
+    static_assert(CQA_MAX_DENSE_SPLITS < (1 << UNIT_SHIFT), "the ticket is the lower bits of the word");
+    const auto draw = [&] { if (threadIdx.x == 0) s_unit = (int)((unsigned)atomicAdd(counter, 1 << UNIT_SHIFT) >> UNIT_SHIFT); };
+    draw();
+    int units_before = 0;
     const long nblk = (num_tokens + BS - 1) / BS, bps = (nblk + ds - 1) / ds;
     int loaded = (int)blockIdx.y;
 #pragma unroll 1
@@ -1010,7 +1020,9 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
         __syncthreads();
         const int n_groups = s_count;
 #pragma unroll 1
-        for (int u = id; u < n_groups * ds; u += n_ctas) {
+        for (;;) {
+            const int u = s_unit - units_before;
+            if (u >= n_groups * ds) break;
             const int at = s_group[u % n_groups], chunk = u / n_groups, y = g0 + at;
             const unsigned heads = s_heads[at];
             const int dkv = y / SUBS, dh0 = dkv * G + (y % SUBS) * HG;
@@ -1039,14 +1051,17 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
                 __syncwarp();
             }
             __syncthreads();
+            draw();
             W.store(sm_m, sm_l, sm_acc, warp);
             cta_merge_store<HG>(sm_m, sm_l, sm_acc, ws.dense_m, ws.dense_l, ws.dense_acc, dh0, chunk, ds);
-            if (take_ticket(ws.tickets + c.kv_heads + dh0, ds, &s_flag))
+            if (take_ticket(ws.tickets + c.kv_heads + dh0, ds, &s_flag, (1 << UNIT_SHIFT) - 1))
                 final_merge(ws.dense_m, ws.dense_l, ws.dense_acc, ds, dh0, HG, ws, true, reinterpret_cast<float *>(ring), c.kv_heads,
                             c.kv_heads * G, __popc(heads));
             __syncthreads();      // the ring is merge scratch
         }
+        units_before += n_groups * ds;
     }
+    if (threadIdx.x == 0 && s_unit == units_before + n_ctas - 1) atomicSub(counter, (units_before + n_ctas) << UNIT_SHIFT);
 }
 
 template <int G, typename T2>
