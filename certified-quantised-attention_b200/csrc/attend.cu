@@ -158,9 +158,9 @@ struct AttLayout {
     static constexpr int RING = ATT_WARPS * ATT_STAGES * STAGE;
     // cross-warp merge buffers and final-merge scratch (both alias the ring)
     static constexpr int MERGE_A = ATT_WARPS * HG * (D + 2) * 4;
-    static constexpr int MERGE_B = (2 * G * CQA_MAX_SPLITS + G + 4 + ATT_WARPS * D) * 4;
-    static constexpr int MERGE_D = (2 * HG * CQA_MAX_DENSE_SPLITS + HG + 4 + ATT_WARPS * D) * 4;
-    static constexpr int MERGE = MERGE_A > MERGE_B ? (MERGE_A > MERGE_D ? MERGE_A : MERGE_D) : (MERGE_B > MERGE_D ? MERGE_B : MERGE_D);
+    static constexpr int MERGE_SPLITS = CQA_MAX_SPLITS > CQA_MAX_DENSE_SPLITS ? CQA_MAX_SPLITS : CQA_MAX_DENSE_SPLITS;
+    static constexpr int MERGE_B = (ATT_WARPS * MERGE_SPLITS + ATT_WARPS + ATT_WARPS * D) * 4;
+    static constexpr int MERGE = MERGE_A > MERGE_B ? MERGE_A : MERGE_B;
     static constexpr int RING_BYTES = RING > MERGE ? RING : MERGE;
     // the query as matrix fragments: [pieces 0,1 | piece 2][8 steps][32 lanes] words of two 16-bit pairs; with float32
     // Tier-2 rows the query rows themselves, and a weight tile per warp
@@ -605,23 +605,26 @@ __device__ __forceinline__ void cta_merge_store(const float *sm_m, const float *
     }
 }
 
-// Final merge of `ns` split partials of heads [head0, head0+nh) by the last CTA to arrive.
-// All 256 threads take part; `sm` is 16-byte aligned scratch of at least 2*nh*ns + nh + 3 + 8*128 floats.
+// Final merge of `ns` split partials of heads [head0, head0+nh) by the last CTA to arrive; bit i of `flagged`: head
+// head0 + i is recomputed densely.  All 256 threads take part; `sm` is 16-byte aligned scratch of at least
+// 8 * ns + 8 + 8*128 floats that no thread uses any more.
 // A thread owns one float4 column of one head and every (256 / (32*nh))-th split.  Its accumulator rows are
-// requested first (up to 20 loads in flight per thread) together with the (m, l) partials, which go through shared
-// memory and which one warp per head turns into per-split scales; the rows are then
-// scaled and summed, the per-thread sums combined through shared memory, normalised and written.
+// requested first (up to 20 loads in flight per thread) together with the (m, l) partials, which every warp turns into
+// the per-split scales of its head by itself; the rows are then scaled and summed, the per-thread sums combined
+// through shared memory, normalised and written.  (A chain of latencies, about 2 us; with the scales made by one warp
+// per head between two CTA barriers and the flags read at the end, it and the ticket took 5 us of a 12 us kernel at
+// 8192 tokens.)
 __device__ __forceinline__ void final_merge(const float *pm, const float *pl, const float *pa, int ns, int head0,
-                                            int nh, const cqa_workspace &ws, bool dense_role, float *sm, int kv_heads, int n_heads_total,
-                                            int arrivals = 1)
+                                            int nh, const cqa_workspace &ws, bool dense_role, unsigned flagged, float *sm, int kv_heads,
+                                            int n_heads_total, int arrivals = 1)
 {
     constexpr int BATCH = 20;
     const bool push_c = ws.partial_out != nullptr && ws.peer_world > 0 && ws.peer_partial[0] != nullptr;
-    float *s_m = sm, *s_sc = sm + nh * ns, *s_l = s_sc + nh * ns;
-    float *s_part = sm + ((2 * nh * ns + nh + 3) & ~3);  // 16-byte aligned for float4 stores
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float *s_sc = sm + warp * ns, *s_part = sm + ((ATT_WARPS * ns + 3) & ~3), *s_l = s_part + ATT_WARPS * D;
     const int nparts = ATT_WARPS / nh;      // nh is 1, 2, 4 or 8
     const int g = warp / nparts, part = warp % nparts;
+    const float *gm = pm + (long)(head0 + g) * ns, *gl = pl + (long)(head0 + g) * ns;
     const float4 *rows = reinterpret_cast<const float4 *>(pa + (long)(head0 + g) * ns * D) + lane;
     float4 buf[BATCH];
     const auto load_rows = [&](int first) {
@@ -631,48 +634,47 @@ __device__ __forceinline__ void final_merge(const float *pm, const float *pl, co
             buf[j] = sp < ns ? __ldcg(rows + (long)sp * (D / 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
-    float m_first = 0.0f, l_first = 0.0f;
-    if (tid < nh * ns) { m_first = __ldcg(pm + (long)head0 * ns + tid); l_first = __ldcg(pl + (long)head0 * ns + tid); }
+    const auto load_ml = [&](int sp, float &m, float &l) {
+        m = sp < ns ? __ldcg(gm + sp) : -INFINITY;
+        l = sp < ns ? __ldcg(gl + sp) : 0.0f;
+    };
+    float m0, l0, m1, l1, M, lsum;
+    load_ml(lane, m0, l0);
+    load_ml(lane + 32, m1, l1);
     load_rows(0);
-    __syncthreads();   // the scratch may still be in use as merge buffers
-    if (tid < nh * ns) { s_m[tid] = m_first; s_sc[tid] = l_first; }
-    for (int i = tid + ATT_THREADS; i < nh * ns; i += ATT_THREADS) {
-        s_m[i] = __ldcg(pm + (long)head0 * ns + i);
-        s_sc[i] = __ldcg(pl + (long)head0 * ns + i);
+    M = fmaxf(m0, m1);
+#pragma unroll 1
+    for (int sp = lane + 64; sp < ns; sp += 32) M = fmaxf(M, __ldcg(gm + sp));
+    M = warp_max(M);
+    const auto scale_of = [&](int sp, float m) {
+        const float sc = m == -INFINITY ? 0.0f : fexp(m - M);
+        if (sp < ns) s_sc[sp] = sc;
+        return sc;
+    };
+    lsum = fmaf(l1, scale_of(lane + 32, m1), l0 * scale_of(lane, m0));
+#pragma unroll 1
+    for (int sp = lane + 64; sp < ns; sp += 32) {
+        float m, l;
+        load_ml(sp, m, l);
+        lsum = fmaf(l, scale_of(sp, m), lsum);
     }
-    __syncthreads();
-    if (warp < nh) {
-        float M = -INFINITY;
-        for (int sp = lane; sp < ns; sp += 32) M = fmaxf(M, s_m[warp * ns + sp]);
-        M = warp_max(M);
-        float lsum = 0.0f;
-        for (int sp = lane; sp < ns; sp += 32) {
-            const float mi = s_m[warp * ns + sp];
-            const float sc = mi == -INFINITY ? 0.0f : fexp(mi - M);
-            lsum = fmaf(s_sc[warp * ns + sp], sc, lsum);
-            s_sc[warp * ns + sp] = sc;
-        }
-        lsum = warp_sum(lsum);
-        if (lane == 0) {
-            s_l[warp] = lsum;
-            if (ws.partial_out != nullptr) {
-                const int h = head0 + warp;
-                const bool flagged = ws.cert != nullptr && (ws.cert[h].dense || ws.any_flags[2]);
-                if (flagged == dense_role) {
-                    if (push_c) {
-                        for (int p = 0; p < ws.peer_world; ++p) {
-                            ws.peer_partial[p][(long)h * CQA_PARTIAL_STRIDE] = M;
-                            ws.peer_partial[p][(long)h * CQA_PARTIAL_STRIDE + 1] = lsum;
-                        }
-                    } else {
-                        ws.partial_out[(long)h * CQA_PARTIAL_STRIDE] = M;
-                        ws.partial_out[(long)h * CQA_PARTIAL_STRIDE + 1] = lsum;
-                    }
+    lsum = warp_sum(lsum);
+    if (lane == 0 && part == 0) {
+        s_l[g] = lsum;
+        if (ws.partial_out != nullptr && (((flagged >> g) & 1u) != 0) == dense_role) {
+            const int h = head0 + g;
+            if (push_c) {
+                for (int p = 0; p < ws.peer_world; ++p) {
+                    ws.peer_partial[p][(long)h * CQA_PARTIAL_STRIDE] = M;
+                    ws.peer_partial[p][(long)h * CQA_PARTIAL_STRIDE + 1] = lsum;
                 }
+            } else {
+                ws.partial_out[(long)h * CQA_PARTIAL_STRIDE] = M;
+                ws.partial_out[(long)h * CQA_PARTIAL_STRIDE + 1] = lsum;
             }
         }
     }
-    __syncthreads();
+    __syncwarp();
     float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 1
     for (int first = 0; first < ns; first += BATCH * nparts) {
@@ -681,7 +683,7 @@ __device__ __forceinline__ void final_merge(const float *pm, const float *pl, co
         for (int j = 0; j < BATCH; ++j) {
             const int sp = first + part + j * nparts;
             if (sp < ns) {
-                const float sc = s_sc[g * ns + sp];
+                const float sc = s_sc[sp];
                 a.x = fmaf(buf[j].x, sc, a.x);
                 a.y = fmaf(buf[j].y, sc, a.y);
                 a.z = fmaf(buf[j].z, sc, a.z);
@@ -693,8 +695,7 @@ __device__ __forceinline__ void final_merge(const float *pm, const float *pl, co
     __syncthreads();
     for (int item = tid; item < nh * D; item += ATT_THREADS) {
         const int gg = item / D, ch = item % D, h = head0 + gg;
-        const bool flagged = ws.cert != nullptr && (ws.cert[h].dense || ws.any_flags[2]);
-        if (flagged != dense_role) continue;
+        if ((((flagged >> gg) & 1u) != 0) != dense_role) continue;
         float acc = 0.0f;
         for (int p = 0; p < nparts; ++p) acc += s_part[(gg * nparts + p) * D + ch];
         if (ws.partial_out != nullptr) {
@@ -734,8 +735,8 @@ __device__ __forceinline__ bool take_ticket(int *ticket, int total, int *s_flag,
         __threadfence();                  // the barrier before it orders the CTA's partials
         const int last = (atomicAdd(ticket, 1) & mask) == total - 1 ? 1 : 0;
         if (last) {
-            atomicSub(ticket, total);     // ready for the next launch
             __threadfence();
+            atomicSub(ticket, total);     // ready for the next launch
         }
         *s_flag = last;
     }
@@ -887,11 +888,12 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
     const bool dense_on = ws.dense_splits > 0 && ws.cert != nullptr;
     const bool dense_all = dense_on && ws.any_flags[2] != 0;
     const int n_dense = dense_all ? c.kv_heads * G : (dense_on ? ws.any_flags[4] : 0);
-    unsigned skip = 0;
-    if (n_dense > 0) {
-        const int f = lane < HG ? (dense_all || ws.cert[head0 + lane].dense) : 0;
-        skip = __ballot_sync(FULL, f != 0);
+    unsigned flagged = 0;        // of the KV head's G heads; without the dense pass their rows are another call's
+    if (n_dense > 0 || (ws.cert != nullptr && !dense_on)) {
+        const int f = lane < G ? (ws.any_flags[2] != 0 || ws.cert[kv * G + lane].dense) : 0;
+        flagged = __ballot_sync(FULL, f != 0);
     }
+    const unsigned skip = dense_on ? (flagged >> (sub * HG)) & ((1u << HG) - 1u) : 0u;
 
     // Lane j keeps the key / value promotion bits of the warp's unit (it0 + j), one bit per head; they are re-read every
     // 32 units.
@@ -972,7 +974,7 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
         W.store(sm_m, sm_l, sm_acc, warp);
         cta_merge_store<HG>(sm_m, sm_l, sm_acc, ws.part_m, ws.part_l, ws.part_acc, head0, split, ns);
         if (take_ticket(ws.tickets + kv, ns * SUBS, &s_flag))
-            final_merge(ws.part_m, ws.part_l, ws.part_acc, ns, kv * G, G, ws, false, reinterpret_cast<float *>(ring), c.kv_heads,
+            final_merge(ws.part_m, ws.part_l, ws.part_acc, ns, kv * G, G, ws, false, flagged, reinterpret_cast<float *>(ring), c.kv_heads,
                         c.kv_heads * G);
     }
     if (n_dense == 0) return;
@@ -1055,7 +1057,7 @@ __device__ __forceinline__ void attend_body(const cqa_cache &c, const cqa_worksp
             W.store(sm_m, sm_l, sm_acc, warp);
             cta_merge_store<HG>(sm_m, sm_l, sm_acc, ws.dense_m, ws.dense_l, ws.dense_acc, dh0, chunk, ds);
             if (take_ticket(ws.tickets + c.kv_heads + dh0, ds, &s_flag, (1 << UNIT_SHIFT) - 1))
-                final_merge(ws.dense_m, ws.dense_l, ws.dense_acc, ds, dh0, HG, ws, true, reinterpret_cast<float *>(ring), c.kv_heads,
+                final_merge(ws.dense_m, ws.dense_l, ws.dense_acc, ds, dh0, HG, ws, true, heads, reinterpret_cast<float *>(ring), c.kv_heads,
                             c.kv_heads * G, __popc(heads));
             __syncthreads();      // the ring is merge scratch
         }
