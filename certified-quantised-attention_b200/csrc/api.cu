@@ -31,7 +31,7 @@ void note_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
 int score_blocks_launch(const cqa_cache *c, const void *q, int q_dtype, long nq, float q_scale, float *m_b,
                         float *s_b, long ld, float *tok, cudaStream_t st, int32_t *zero_words, int n_zero_words,
-                        const ScorePush *push);
+                        const ScorePush *push, long early_blocks = 0);
 int select_launch(const cqa_cache *c, const cqa_knobs *kn, const cqa_workspace *ws, long nq, long nact,
                   const float *u, long u_ld, cudaStream_t st);
 int certify_launch(const cqa_cache *c, const cqa_knobs *kn, const cqa_workspace *ws, const void *q, int q_dtype,
@@ -136,6 +136,15 @@ extern "C" int cqa_certify(const cqa_cache *c, const cqa_knobs *knobs, const cqa
     return certify_launch(c, knobs, ws, q, q_dtype, nq, nact, (cudaStream_t)stream);
 }
 
+// early_blocks > 0: the launch before on this stream was cqa_append_token of this cache, it changed no block below and no
+// channel maximum, and q was written before it.
+static int layer_step(const cqa_cache *c, const cqa_knobs *knobs, const cqa_workspace *ws, const void *q, int q_dtype,
+                      int64_t num_tokens, int64_t nq, const float *exploration_u, int64_t u_ld, void *stream, long early_blocks);
+
+// Blocks that may be scored while the token at `pos` is appended: all complete ones, unless the token completes one (that
+// also raises the channel maxima, which the selector reads before it waits).
+static long early_blocks_of(int64_t pos) { return pos % BS == BS - 1 ? 0 : (long)(pos / BS); }
+
 static int decode_step_host(const cqa_cache *c, const cqa_knobs *knobs, const cqa_workspace *ws, const void *qkv_host,
                             void *qkv_dev, int dtype, int64_t pos, int defer_int4, float *out_host, void *stream,
                             bool wait)
@@ -164,7 +173,7 @@ static int decode_step_host(const cqa_cache *c, const cqa_knobs *knobs, const cq
         w.out = static_cast<float *>(mapped);
     else
         (void)cudaGetLastError();
-    rc = cqa_layer_step(c, knobs, &w, q, dtype, num_tokens, num_tokens / BS, nullptr, 0, stream);
+    rc = layer_step(c, knobs, &w, q, dtype, num_tokens, num_tokens / BS, nullptr, 0, stream, early_blocks_of(pos));
     if (rc) return rc;
     if (w.out == ws->out)
         rc = check_cuda(cudaMemcpyAsync(out_host, ws->out, H * D * sizeof(float), cudaMemcpyDeviceToHost, st), "copy of the output");
@@ -184,6 +193,21 @@ extern "C" int cqa_decode_step_host_async(const cqa_cache *c, const cqa_knobs *k
                                           float *out_host, void *stream)
 {
     return decode_step_host(c, knobs, ws, qkv_host, qkv_dev, dtype, pos, defer_int4, out_host, stream, false);
+}
+
+// The attention rows of up to 64 layers into mapped host memory, 16 bytes per thread.  Bound by the link (128 KB: about
+// 3 us).  Phase 2 wrote its rows there itself before; every layer's kernel then ended with a flush across the link, and
+// the next layer waited for it (eight layers of 32768 tokens, 32 heads: 521 us a token, 499 so).
+constexpr int OUT_ROWS = 64;
+struct OutRows {
+    const float *src[OUT_ROWS];
+    float *dst[OUT_ROWS];
+};
+__global__ void __launch_bounds__(256) out_rows_kernel(const __grid_constant__ OutRows rows, int quads)
+{
+    grid_dependency_wait();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < quads) reinterpret_cast<float4 *>(rows.dst[blockIdx.y])[i] = __ldcg(reinterpret_cast<const float4 *>(rows.src[blockIdx.y]) + i);
 }
 
 extern "C" int cqa_decode_token_host(const cqa_layer_call *layers, int n_layers, const cqa_knobs *knobs, void *qkv_dev,
@@ -222,26 +246,54 @@ extern "C" int cqa_decode_token_host(const cqa_layer_call *layers, int n_layers,
         if (rc) return rc;
         l = r;
     }
+    // The rows go to the host behind the last layer: by one kernel per 64 layers where the driver maps the caller's
+    // pinned buffer for the device, by a copy per layer otherwise.  Layers that share output rows send theirs at once.
+    bool shared = false;
+    for (int l = 0; l < n_layers && !shared; ++l)
+        for (int k = 0; k < l; ++k) shared |= layers[k].ws->out == layers[l].ws->out;
+    const auto send = [&](int first, int end) {
+        for (int l = first; l < end;) {
+            OutRows rows;
+            int n = 0;
+            for (; n < OUT_ROWS && l + n < end; ++n) {
+                void *mapped = nullptr;
+                if (cudaHostGetDevicePointer(&mapped, layers[l + n].out_host, 0) != cudaSuccess || mapped == nullptr) {
+                    (void)cudaGetLastError();
+                    break;
+                }
+                if ((((uintptr_t)mapped | (uintptr_t)layers[l + n].ws->out) & 15) != 0) break;
+                rows.src[n] = layers[l + n].ws->out;
+                rows.dst[n] = static_cast<float *>(mapped);
+            }
+            int rc;
+            if (n > 0) {
+                const int quads = (int)(H * D / 4);
+                rc = check_cuda(launch_chained(out_rows_kernel, dim3((unsigned)((quads + 255) / 256), (unsigned)n), dim3(256), 0, st, true,
+                                               rows, quads), "out_rows_kernel");
+            } else {
+                rc = check_cuda(cudaMemcpyAsync(layers[l].out_host, layers[l].ws->out, H * D * sizeof(float), cudaMemcpyDeviceToHost, st),
+                                "copy of the output");
+                n = 1;
+            }
+            if (rc) return rc;
+            l += n;
+        }
+        return (int)CQA_OK;
+    };
     for (int l = 0; l < n_layers; ++l) {
         const cqa_layer_call &c = layers[l];
-        // Phase 2 writes its rows straight into the caller's pinned buffer when the driver maps it for the device
-        cqa_workspace w = *c.ws;
-        void *mapped = nullptr;
-        if (cudaHostGetDevicePointer(&mapped, c.out_host, 0) == cudaSuccess && mapped != nullptr)
-            w.out = static_cast<float *>(mapped);
-        else
-            (void)cudaGetLastError();
         const char *in = dev + (size_t)l * row;
         int rc = cqa_append_token(c.cache, in + H * D * esz, in + (H + KV) * D * esz, dtype, c.pos, c.defer_int4, stream);
         if (rc) return rc;
         const int64_t num_tokens = c.pos + 1;
-        rc = cqa_layer_step(c.cache, knobs, &w, in, dtype, num_tokens, num_tokens / BS, nullptr, 0, stream);
+        rc = layer_step(c.cache, knobs, c.ws, in, dtype, num_tokens, num_tokens / BS, nullptr, 0, stream, early_blocks_of(c.pos));
         if (rc) return rc;
-        if (w.out == c.ws->out) {
-            rc = check_cuda(cudaMemcpyAsync(c.out_host, c.ws->out, H * D * sizeof(float), cudaMemcpyDeviceToHost, st),
-                            "copy of the output");
-            if (rc) return rc;
-        }
+        if (shared) rc = send(l, l + 1);
+        if (rc) return rc;
+    }
+    if (!shared) {
+        const int rc = send(0, n_layers);
+        if (rc) return rc;
     }
     return check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize");
 }
@@ -322,9 +374,8 @@ extern "C" int cqa_attend_static(const cqa_cache *c, const cqa_workspace *ws, co
                                 (cudaStream_t)stream);
 }
 
-extern "C" int cqa_layer_step(const cqa_cache *c, const cqa_knobs *knobs, const cqa_workspace *ws, const void *q,
-                              int q_dtype, int64_t num_tokens, int64_t nq, const float *exploration_u,
-                              int64_t u_ld, void *stream)
+static int layer_step(const cqa_cache *c, const cqa_knobs *knobs, const cqa_workspace *ws, const void *q, int q_dtype,
+                      int64_t num_tokens, int64_t nq, const float *exploration_u, int64_t u_ld, void *stream, long early_blocks)
 {
     // every argument check comes before the first launch: a bad call must not write anything on the device
     int rc = check_common(c, ws, "cqa_layer_step");
@@ -352,11 +403,18 @@ extern "C" int cqa_layer_step(const cqa_cache *c, const cqa_knobs *knobs, const 
     if (rc) return rc;
     const int n_flag_words = 5 + c->kv_heads * c->gqa_group;
     rc = score_blocks_launch(c, q, q_dtype, nq, knobs->q_scale, ws->m_b, ws->s_b, ws->ld, ws->token_scores, st,
-                             ws->any_flags, n_flag_words, nullptr);
+                             ws->any_flags, n_flag_words, nullptr, early_blocks);
     if (rc) return rc;
     rc = selcert_launch(c, knobs, ws, q, q_dtype, nq, nact, exploration_u, u_ld, 3 | 16, st);   // select + certify in one launch; flags cleared by the score kernel
     if (rc) return rc;
     return attend_launch(c, ws, q, q_dtype, nq, nact, num_tokens, last_valid, knobs->q_scale, st, true);
+}
+
+extern "C" int cqa_layer_step(const cqa_cache *c, const cqa_knobs *knobs, const cqa_workspace *ws, const void *q,
+                              int q_dtype, int64_t num_tokens, int64_t nq, const float *exploration_u,
+                              int64_t u_ld, void *stream)
+{
+    return layer_step(c, knobs, ws, q, q_dtype, num_tokens, nq, exploration_u, u_ld, stream, 0);
 }
 
 extern "C" int cqa_layer_step_batched(const cqa_batch_item *items, int n_items, void *items_dev, const cqa_knobs *knobs,

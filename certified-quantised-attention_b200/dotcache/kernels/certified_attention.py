@@ -358,8 +358,8 @@ def certified_decode_token_host(
     """`certified_decode_step_host` for every layer of a model in ONE library call (cqa_decode_token_host):
     `caches` is the list of the layers' caches, `qkv_host` a pinned [L, (H + 2 KV) * 128] tensor, `out_host` a
     pinned float32 [L, H, 128] tensor that holds every layer's attention rows when the call returns.  The loop over
-    the layers runs inside the library, all inputs are copied before the first kernel, Phase 2 writes into `out_host`
-    directly when it is pinned, and the stream is waited for once.  Row l equals what
+    the layers runs inside the library, all inputs are copied before the first kernel, the rows go to `out_host`
+    behind the last layer (by one kernel when it is pinned), and the stream is waited for once.  Row l equals what
     `certified_decode_step_host(caches[l], qkv_host[l], ...)` returns.  An addition (no reference counterpart)."""
     n_layers = len(caches)
     if n_layers == 0:

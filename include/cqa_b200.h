@@ -416,11 +416,12 @@ int cqa_decode_step_host_async(const cqa_cache *c, const cqa_knobs *knobs, const
 
 /* One decode token of a whole model from host buffers: the inputs of all n_layers entries are
  * copied to the device first (qkv_dev holds n_layers rows of (H + 2 KV) * 128 elements), then
- * each layer's append and layer step are queued in order, then ONE wait on the stream.  When
- * out_host is pinned memory that the device can address, Phase 2 writes the rows into it
- * directly (ws->out of that layer is then left untouched); otherwise they are copied.  No
- * transfer sits between two layers' kernels, and the loop over the layers runs inside the
- * library.  knobs and dtype are shared by the layers; all caches share the head geometry. */
+ * each layer's append and layer step are queued in order, then ONE wait on the stream.  The
+ * rows of all layers (ws->out) go to out_host behind the last layer, by one kernel where
+ * out_host is pinned memory that the device can address, otherwise by copies; layers that
+ * share ws->out send theirs at once.  With rows of their own no transfer sits between two
+ * layers' kernels, and the loop over the layers runs inside the library.  knobs and dtype are
+ * shared by the layers; all caches share the head geometry. */
 typedef struct cqa_layer_call {
     const cqa_cache *cache;
     const cqa_workspace *ws;
