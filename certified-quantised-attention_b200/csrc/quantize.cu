@@ -856,7 +856,8 @@ __global__ void __launch_bounds__(128) append_token_batched_kernel(const cqa_bat
 
 // The same with the records as kernel parameters: the CTAs of KV head 0 write them to `dev`, where the other kernels
 // of the step read them.  A copy of the records between two steps cost a transfer through the copy engine in the
-// middle of a chain of kernels.
+// middle of a chain of kernels, about 10 us of a batch step.  Parameters grow the launch itself, hence two sizes; beyond 40
+// sequences the step is long enough for the copy.
 template <int N>
 struct BatchRecords {
     cqa_batch_item it[N];
